@@ -57,8 +57,8 @@ namespace {
 constexpr int kMaxMachines = 255;
 constexpr int kMaxGenes = 8192;     // bitonic sort buffer: 8192 x 8 B = 64 KB shared memory
 constexpr int kMaxSide = 8191;      // 13-bit fields of the selection key
-constexpr int kMaxItemWarps = 4;   // decode CTAs have 1, 2 or 4 warps (one item per CTA)
-constexpr int kGreedyThreads = 128;
+constexpr int kGreedyThreads = 256;
+constexpr int kGreedyCtas = 8;  // CTAs of the greedy's cluster (the portable limit)
 constexpr int kResidentWarps = 32;  // automatic shape: 32 warps per SM (the register limit at 64 per thread)
 constexpr int kMaxInst = BRKGA_MAX_INSTANCES;
 constexpr int kMaxCtasPerSm = 32;
@@ -512,14 +512,15 @@ __global__ void order_items_kernel(const __grid_constant__ Tables tb, const __gr
   for (int i = tid; i < run.n_items; i += nt) run.order[atomicAdd(&start[item_weight(tb, run, i)], 1)] = i;
 }
 
-// Shared state of one CTA-cooperative plate search.
+// Shared state of one plate search by a CTA of kWarps warps.
+template <int kWarps>
 struct SearchShared {
   unsigned long long best;
   int chunk, total, nr;
   int rlist[4];
   int rh[4];      // heights of the rotations in rlist
   RotDev rd[4];   // their descriptors, read by every chunk
-  unsigned char surv[kMaxItemWarps][32];  // per warp: lanes whose candidate passed the vacancy filter
+  unsigned char surv[kWarps][32];  // per warp: lanes whose candidate passed the vacancy filter
 };
 
 // Best placement key of part type t (absolute) on one plate (kKeyNone if it
@@ -528,10 +529,11 @@ struct SearchShared {
 // skip chunks that cannot beat the best key found so far, stop once no
 // rotation can at the current level, and merge with atomicMin.  Called by
 // all threads of the CTA; contains __syncthreads.
+template <int kWarps>
 __device__ __forceinline__ unsigned long long search_plate(const Tables& tb, const MachDev& md,
                                                            const uint32_t* grid, const uint16_t* vac, int enc,
                                                            int t, const RotList* rlp, int task_max, int32_t* status,
-                                                           SearchShared& sh,
+                                                           SearchShared<kWarps>& sh,
                                                            unsigned long long& c_tests,
                                                            unsigned long long& c_chunks,
                                                            unsigned long long& c_bytes) {
@@ -826,7 +828,7 @@ __global__ void __launch_bounds__(kThreads, kResidentWarps * 32 / kThreads)
   // from is not written again until the search after next, by which time every
   // thread has passed the next search's barriers — so a search needs no
   // barrier after reading its result.
-  __shared__ SearchShared sh2[2];
+  __shared__ SearchShared<kThreads / 32> sh2[2];
   __shared__ ItemCtx ctx;
   int sh_par = 0;
   __shared__ int s_fail, s_pool;
@@ -997,17 +999,31 @@ __global__ void reduce_kernel(const __grid_constant__ Tables tb, const __grid_co
 }
 
 // Greedy initial solution (BRKGA_alg3.py:445-603 with binClassInitialSol.py):
-// one CTA walks the parts in the given order; each part goes where the
-// system makespan after placing it is smallest (ties: the later option wins
-// over an earlier one on another machine or a new plate, the first existing
-// plate wins within a machine): a new plate on some machine (best rotation at
-// column 0, bottom row L-1) or any existing plate of the machine that can take
-// it (every plate is tested, no area filter).  Plates live in the global pool.
+// the parts go in the given order, each where the system makespan after
+// placing it is smallest (ties: the later option wins over an earlier one on
+// another machine or a new plate, the first existing plate wins within a
+// machine): a new plate on some machine (best rotation at column 0, bottom row
+// L-1) or any existing plate of the machine that can take it (every plate is
+// tested, no area filter).
+//
+// A part's plate searches are independent and are most of the work, so one
+// cluster of kGreedyCtas CTAs shares them: plate b belongs to CTA
+// b % kGreedyCtas, which alone reads and writes its grid and scalars (in the
+// global pool) and sends every search's key to the other CTAs' shared memory.
+// After one cluster barrier per part each CTA has all keys and takes the same
+// decision from its own copy of the makespans and of the plates' height times;
+// the chosen plate's owner inserts the part while the others go on to the next
+// one (the keys of alternate parts have buffers of their own, so none is
+// overwritten before every CTA has read it).  What bounds it is the latency of
+// one search and one insertion per part: the call took 7.4 ms on one CTA of
+// four warps and takes 2.4 ms here at 100 parts on four machines (P100M4),
+// 17.4 and 4.9 ms at 200 parts on six (P200M6), 1.34 and 0.94 ms at 50 parts
+// on two (P50M2); with four warps per CTA 2.9, 5.5 and 1.05 ms, with sixteen
+// 2.35, 4.9 and 0.93 ms.
 // Single-instance problems only, so every table base is 0.
 struct GreedyArgs {
   int N, M, T;
   int32_t* status;
-  unsigned long long* counters;
   BinScal* binscal;
   uint32_t* pool;
   int slot_words, slot_vac_off;
@@ -1015,115 +1031,177 @@ struct GreedyArgs {
   int n;
   int32_t* out_machine;  // [n]
   BrkgaPlacement* out;   // [n]: gene, plate index within its machine, x, bottom row y, rotation
-  int32_t* plate_machine;
-  int32_t* plate_index;  // index of the plate within its machine
+  int32_t* plate_index;  // [n]: index of the plate within its machine
   double* machine_makespan;  // [M]
+  unsigned char* state;      // the CTAs' state in global memory, state_bytes each, or NULL: in shared memory
+  size_t state_bytes;
 };
+
+// A CTA's state: per plate the keys of two parts, its largest height time and
+// its machine's next plate; per machine its makespan, its first and last plate
+// and their number.  In shared memory as long as it fits (up to some 8,000 parts).
+size_t greedy_state_bytes(int n, int M) { return (size_t)n * 28 + (size_t)M * 20; }
+constexpr size_t kGreedyMaxSmem = 229 * 1024;
+
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+
+// All threads of all CTAs of the cluster; shared-memory writes before it, remote ones too, are seen after it.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// Store to the same shared variable of CTA `rank` of the cluster.
+__device__ __forceinline__ void cluster_store(unsigned long long* p, unsigned rank, unsigned long long v) {
+  const unsigned local = (unsigned)__cvta_generic_to_shared(p);
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.u64 [a], %2;\n\t}" ::"r"(local),
+               "r"(rank), "l"(v)
+               : "memory");
+}
 
 __global__ void __launch_bounds__(kGreedyThreads) greedy_kernel(const __grid_constant__ Tables tb,
                                                                 const __grid_constant__ GreedyArgs g) {
-  __shared__ SearchShared sh2[2];  // alternate searches, as in decode_kernel
-  __shared__ int s_fail;
+  extern __shared__ __align__(16) unsigned char gsm[];
+  const unsigned rank = cluster_rank();
+  unsigned char* state = g.state ? g.state + rank * g.state_bytes : gsm;
+  unsigned long long* keys = reinterpret_cast<unsigned long long*>(state);  // [2][n]
+  double* pth = reinterpret_cast<double*>(keys + 2 * (size_t)g.n);
+  double* makespan = pth + g.n;
+  int* next = reinterpret_cast<int*>(makespan + g.M);
+  int* first = next + g.n;
+  int* last = first + g.M;
+  int* count = last + g.M;
+  __shared__ SearchShared<kGreedyThreads / 32> sh2[2];  // alternate searches, as in decode_kernel
+  struct Choice {
+    int machine, plate;  // plate -1: a new one, machine -1: the part fits nowhere
+    unsigned long long key;
+    double cand;
+  };
+  __shared__ Choice choice;
   int sh_par = 0;
   const int tid = threadIdx.x;
   BinScal* bs = g.binscal;
-  unsigned long long c_tests = 0, c_chunks = 0, c_bytes = 0;
+  unsigned long long c_tests = 0, c_chunks = 0, c_bytes = 0;  // of search_plate, not reported here
   int nplates = 0;
   double cw = 0.0;  // current_worst_makespan
-  for (int m = tid; m < g.M; m += kGreedyThreads) g.machine_makespan[m] = 0.0;
-  __syncthreads();
+  for (int m = tid; m < g.M; m += kGreedyThreads) {
+    makespan[m] = 0.0;
+    first[m] = last[m] = -1;
+    count[m] = 0;
+  }
+  // Plate b lives in pool slot b, so bs[b].pool is free to hold its machine.
+  cluster_sync();
   for (int k = 0; k < g.n; ++k) {
     const int gene = g.order[k];
     const int t = tb.gene_type[gene];
     const double a = tb.part_area[t];
-    double best = INFINITY;
-    int kind = -1, cm = -1, cb = -1;  // kind 0 = new plate, 1 = existing plate
-    unsigned long long ckey = kKeyNone;
-    double ccand = 0.0;
-    for (int m = 0; m < g.M; ++m) {
-      bool placed_in_exist = false;
-      if (!tb.fits[t * g.M + m]) continue;  // BRKGA_alg3.py:465-470
+    unsigned long long* kk = keys + (size_t)(k & 1) * g.n;
+    for (int b = (int)rank; b < nplates; b += kGreedyCtas) {
+      const int m = bs[b].pool;
       const MachDev md = tb.mach[m];
-      const double mm = g.machine_makespan[m];
-      const double ptm = tb.pt[(size_t)m * g.T + t], pthm = tb.pth[(size_t)m * g.T + t];
-      const double cand = ((mm + md.setup) + ptm) + pthm;  // :472
-      const double nm = cw > cand ? cw : cand;
-      if (nm <= best) {
-        best = nm;
-        kind = 0;
-        cm = m;
-        ccand = cand;
-      }
-      for (int b = 0; b < nplates; ++b) {
-        if (g.plate_machine[b] != m) continue;
-        const uint32_t* grid = g.pool + (size_t)bs[b].pool * g.slot_words;
-        const unsigned long long key =
-            search_plate(tb, md, grid, reinterpret_cast<const uint16_t*>(grid + g.slot_vac_off), bs[b].enc, t,
-                         tb.rl + (size_t)t * g.M + m, kDefaultTaskMax, g.status, sh2[sh_par], c_tests, c_chunks,
-                         c_bytes);
+      unsigned long long key = kKeyNone;
+      if (tb.fits[t * g.M + m]) {  // BRKGA_alg3.py:465-470
+        const uint32_t* grid = g.pool + (size_t)b * g.slot_words;
+        key = search_plate(tb, md, grid, reinterpret_cast<const uint16_t*>(grid + g.slot_vac_off), bs[b].enc, t,
+                           tb.rl + (size_t)t * g.M + m, kDefaultTaskMax, g.status, sh2[sh_par], c_tests, c_chunks,
+                           c_bytes);
         sh_par ^= 1;
-        if (key == kKeyNone) continue;
-        const double bpth = bs[b].pth;
-        const double cand2 = bpth < pthm ? ((mm - bpth) + pthm) + ptm : mm + ptm;  // :486-489
-        const double nm2 = cw > cand2 ? cw : cand2;
-        if (nm2 <= best) {
-          if (placed_in_exist && nm2 == best) continue;
-          placed_in_exist = true;
-          best = nm2;
-          kind = 1;
-          cm = m;
-          cb = b;
-          ckey = key;
-          ccand = cand2;
+      }
+      if (tid < kGreedyCtas) {
+        if (g.state) reinterpret_cast<unsigned long long*>(g.state + tid * g.state_bytes)[(size_t)(k & 1) * g.n + b] = key;
+        else cluster_store(&kk[b], (unsigned)tid, key);
+      }
+    }
+    cluster_sync();
+    if (tid == 0) {
+      Choice best{-1, -1, kKeyNone, 0.0};
+      double bv = INFINITY;
+      for (int m = 0; m < g.M; ++m) {
+        if (!tb.fits[t * g.M + m]) continue;
+        bool placed_in_exist = false;
+        const double mm = makespan[m];
+        const double ptm = tb.pt[(size_t)m * g.T + t], pthm = tb.pth[(size_t)m * g.T + t];
+        const double cand = ((mm + tb.mach[m].setup) + ptm) + pthm;  // :472
+        const double nm = cw > cand ? cw : cand;
+        if (nm <= bv) {
+          bv = nm;
+          best = Choice{m, -1, kKeyNone, cand};
+        }
+        for (int b = first[m]; b >= 0; b = next[b]) {
+          if (kk[b] == kKeyNone) continue;
+          const double cand2 = pth[b] < pthm ? ((mm - pth[b]) + pthm) + ptm : mm + ptm;  // :486-489
+          const double nm2 = cw > cand2 ? cw : cand2;
+          if (nm2 <= bv) {
+            if (placed_in_exist && nm2 == bv) continue;
+            placed_in_exist = true;
+            bv = nm2;
+            best = Choice{m, b, kk[b], cand2};
+          }
+        }
+      }
+      choice = best;
+      if (best.machine >= 0) {
+        const int m = best.machine;
+        const double pthm = tb.pth[(size_t)m * g.T + t];
+        makespan[m] = best.cand;  // :541, :565
+        if (best.plate < 0 && nplates < g.n) {
+          const int b = nplates;
+          next[b] = -1;
+          if (last[m] < 0) first[m] = b;
+          else next[last[m]] = b;
+          last[m] = b;
+          if (b % kGreedyCtas == (int)rank) g.plate_index[b] = count[m];
+          ++count[m];
+          pth[b] = pthm > 0.0 ? pthm : 0.0;
+        } else if (best.plate >= 0 && pthm > pth[best.plate]) {
+          pth[best.plate] = pthm;
         }
       }
     }
-    if (kind < 0) {  // fits no machine: the reference crashes here (bestBatch == [])
-      if (tid == 0) raise_status(g.status, BRKGA_ERR_BAD_INSTANCE);
+    __syncthreads();
+    const Choice c = choice;
+    // The same decision in every CTA, so all of them leave here together.
+    if (c.machine < 0) {  // fits no machine: the reference crashes here (bestBatch == [])
+      if (tid == 0 && rank == 0) raise_status(g.status, BRKGA_ERR_BAD_INSTANCE);
       return;
     }
-    const MachDev md = tb.mach[cm];
-    int r, x, ty, b;
-    if (kind == 0) {
-      r = tb.best_rot[t];
-      if (tid == 0) s_fail = (!tb.newbin_ok[t * g.M + cm] || nplates >= g.n) ? 1 : 0;
-      __syncthreads();
-      if (s_fail) {
-        if (tid == 0) raise_status(g.status, BRKGA_ERR_NEW_BIN_UNFIT);
+    const MachDev md = tb.mach[c.machine];
+    int r, x, ty, b = c.plate;
+    const bool fresh = b < 0;
+    if (fresh) {
+      if (!tb.newbin_ok[t * g.M + c.machine] || nplates >= g.n) {
+        if (tid == 0 && rank == 0) raise_status(g.status, BRKGA_ERR_NEW_BIN_UNFIT);
         return;
       }
+      r = tb.best_rot[t];
       b = nplates++;
-      uint32_t* grid = g.pool + (size_t)b * g.slot_words;
-      open_plate(md, grid, reinterpret_cast<uint16_t*>(grid + g.slot_vac_off), &bs[b], b);
-      if (tid == 0) {
-        int idx = 0;
-        for (int q = 0; q < b; ++q) idx += g.plate_machine[q] == cm;
-        g.plate_machine[b] = cm;
-        g.plate_index[b] = idx;
-      }
       x = 0;
       ty = md.L - tb.rot[t * 4 + r].h;
     } else {
       int y;
-      decode_key(ckey, &r, &x, &y);
+      decode_key(c.key, &r, &x, &y);
       ty = y - tb.rot[t * 4 + r].h + 1;
-      b = cb;
     }
-    uint32_t* grid = g.pool + (size_t)bs[b].pool * g.slot_words;
-    place_part(tb, md, grid, reinterpret_cast<uint16_t*>(grid + g.slot_vac_off), &bs[b], t, r, x, ty, a,
-               tb.pt[(size_t)cm * g.T + t], tb.pth[(size_t)cm * g.T + t]);
-    if (tid == 0) {
-      g.out_machine[k] = cm;
-      g.out[k] = BrkgaPlacement{gene, g.plate_index[b], x, ty + tb.rot[t * 4 + r].h - 1, r};
-      g.machine_makespan[cm] = ccand;  // :541, :565
+    cw = cw > c.cand ? cw : c.cand;
+    if ((unsigned)b % kGreedyCtas == rank) {
+      uint32_t* grid = g.pool + (size_t)b * g.slot_words;
+      uint16_t* vac = reinterpret_cast<uint16_t*>(grid + g.slot_vac_off);
+      if (fresh) open_plate(md, grid, vac, &bs[b], c.machine);
+      place_part(tb, md, grid, vac, &bs[b], t, r, x, ty, a, tb.pt[(size_t)c.machine * g.T + t],
+                 tb.pth[(size_t)c.machine * g.T + t]);
+      if (tid == 0) {
+        g.out_machine[k] = c.machine;
+        g.out[k] = BrkgaPlacement{gene, g.plate_index[b], x, ty + tb.rot[t * 4 + r].h - 1, r};
+      }
     }
-    cw = cw > ccand ? cw : ccand;
-    __syncthreads();
+    __syncthreads();  // `choice` is read
   }
-  if (tid == 0) {
-    atomicAdd(&g.counters[0], c_tests);
-    atomicAdd(&g.counters[3], c_bytes);
-  }
+  if (rank == 0)
+    for (int m = tid; m < g.M; m += kGreedyThreads) g.machine_makespan[m] = makespan[m];
+  cluster_sync();  // no CTA leaves while another may still store into its shared memory
 }
 
 // ---------------------------------------------------------------- chunk tests
@@ -1277,6 +1355,9 @@ struct BrkgaProblem {
   int e_cap_P = 0;
   bool e_cap_log = false;
   int64_t e_pool_bins = 0;
+  // brkga_initial_solution_host state
+  void* greedy_ws = nullptr;
+  size_t greedy_bytes = 0;
   int64_t last_counters[4] = {0, 0, 0, 0};
 };
 
@@ -1799,6 +1880,7 @@ void brkga_problem_destroy(BrkgaProblem* pb) {
     if (pb->e_status) cudaFree(pb->e_status);
     if (pb->e_log) cudaFree(pb->e_log);
     if (pb->e_ws) cudaFree(pb->e_ws);
+    if (pb->greedy_ws) cudaFree(pb->greedy_ws);
     if (pb->e_host) cudaFreeHost(pb->e_host);
     if (pb->stream) cudaStreamDestroy(pb->stream);
   }
@@ -2095,7 +2177,7 @@ int brkga_initial_solution_host(BrkgaProblem* pb, const int32_t* h_order, int32_
   std::lock_guard<std::mutex> lock(pb->mu);
   DeviceGuard guard(pb->device);
   const int nn = std::max(n, 1);
-  // one allocation: order, outputs, plate tables, scalars, counters, status, pool (one plate per part at most)
+  // one allocation: order, outputs, plate indices, scalars, status, pool (one plate per part at most), CTA state
   size_t o = 0;
   const size_t off_order = o;
   o = align_up(o + (size_t)nn * 4, 256);
@@ -2103,8 +2185,6 @@ int brkga_initial_solution_host(BrkgaProblem* pb, const int32_t* h_order, int32_
   o = align_up(o + (size_t)nn * 4, 256);
   const size_t off_out = o;
   o = align_up(o + (size_t)nn * sizeof(BrkgaPlacement), 256);
-  const size_t off_pm = o;
-  o = align_up(o + (size_t)nn * 4, 256);
   const size_t off_pi = o;
   o = align_up(o + (size_t)nn * 4, 256);
   const size_t off_mk = o;
@@ -2115,8 +2195,18 @@ int brkga_initial_solution_host(BrkgaProblem* pb, const int32_t* h_order, int32_
   o = align_up(o + 64, 256);
   const size_t off_pool = o;
   o = align_up(o + (size_t)nn * pb->slot_words * 4, 256);
-  char* d = nullptr;
-  if (cudaMalloc(&d, o) != cudaSuccess) return BRKGA_ERR_CUDA;
+  const size_t state_bytes = align_up(greedy_state_bytes(nn, pb->M), 256);
+  const bool in_smem = state_bytes <= kGreedyMaxSmem - 4096;
+  const size_t off_state = o;
+  if (!in_smem) o += kGreedyCtas * state_bytes;
+  if (o > pb->greedy_bytes) {  // kept for the next call on this problem
+    cudaFree(pb->greedy_ws);
+    pb->greedy_ws = nullptr;
+    pb->greedy_bytes = 0;
+    if (cudaMalloc(&pb->greedy_ws, o) != cudaSuccess) return BRKGA_ERR_CUDA;
+    pb->greedy_bytes = o;
+  }
+  char* d = static_cast<char*>(pb->greedy_ws);
   int st = BRKGA_OK;
   do {
     if (cudaMemset(d, 0, off_pool) != cudaSuccess ||
@@ -2130,7 +2220,6 @@ int brkga_initial_solution_host(BrkgaProblem* pb, const int32_t* h_order, int32_
     g.M = pb->M;
     g.T = pb->T;
     g.status = reinterpret_cast<int32_t*>(d + off_ctr + 40);
-    g.counters = reinterpret_cast<unsigned long long*>(d + off_ctr + 8);
     g.binscal = reinterpret_cast<BinScal*>(d + off_bs);
     g.pool = reinterpret_cast<uint32_t*>(d + off_pool);
     g.slot_words = pb->slot_words;
@@ -2139,12 +2228,24 @@ int brkga_initial_solution_host(BrkgaProblem* pb, const int32_t* h_order, int32_
     g.n = n;
     g.out_machine = reinterpret_cast<int32_t*>(d + off_mach);
     g.out = reinterpret_cast<BrkgaPlacement*>(d + off_out);
-    g.plate_machine = reinterpret_cast<int32_t*>(d + off_pm);
     g.plate_index = reinterpret_cast<int32_t*>(d + off_pi);
     g.machine_makespan = reinterpret_cast<double*>(d + off_mk);
-    greedy_kernel<<<1, kGreedyThreads>>>(pb->tb, g);
+    g.state = in_smem ? nullptr : reinterpret_cast<unsigned char*>(d + off_state);
+    g.state_bytes = state_bytes;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = kGreedyCtas;
+    cfg.blockDim = kGreedyThreads;
+    cfg.dynamicSmemBytes = in_smem ? state_bytes : 0;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kGreedyCtas;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
     int32_t status = 0;
-    if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess ||
+    if (cudaFuncSetAttribute(greedy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kGreedyMaxSmem - 4096) != cudaSuccess ||
+        cudaLaunchKernelEx(&cfg, greedy_kernel, pb->tb, g) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess ||
         cudaMemcpy(&status, g.status, 4, cudaMemcpyDeviceToHost) != cudaSuccess) {
       st = BRKGA_ERR_CUDA;
       break;
@@ -2159,7 +2260,6 @@ int brkga_initial_solution_host(BrkgaProblem* pb, const int32_t* h_order, int32_
         cudaMemcpy(h_machine_makespan, g.machine_makespan, (size_t)pb->M * 8, cudaMemcpyDeviceToHost) != cudaSuccess)
       st = BRKGA_ERR_CUDA;
   } while (false);
-  cudaFree(d);
   return st;
 }
 
