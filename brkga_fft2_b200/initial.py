@@ -50,19 +50,19 @@ def encode(machine, place, instance_parts, type_ids, gene_type, nb_machines: int
     inst = np.asarray(instance_parts)
     N = inst.size
     array = np.zeros(2 * N)
-    used = set()
+    free = {}  # genes of each part not yet used, the first one last
+    for idx in range(N - 1, -1, -1):
+        free.setdefault(int(inst[idx]), []).append(idx)
+    genes = place["gene"].tolist()
+    bins = place["bin"].tolist()
+    on = [[] for _ in range(nb_machines)]
+    for k, m in enumerate(np.asarray(machine).tolist()):
+        if 0 <= m < nb_machines:
+            on[m].append(k)
     for m in range(nb_machines):
-        ks = [k for k in range(len(machine)) if machine[k] == m]
-        ks.sort(key=lambda k: (int(place[k]["bin"]), k))  # plates in creation order, parts in insertion order
-        parts_machine = [int(type_ids[gene_type[int(place[k]["gene"])]]) for k in ks]
-        positions = []
-        for value in parts_machine:
-            for idx, val in enumerate(inst):
-                if val == value and idx not in used:
-                    positions.append(idx)
-                    used.add(idx)
-                    break
-        pos = np.array(positions, dtype=np.int64)
+        ks = sorted(on[m], key=lambda k: (bins[k], k))  # plates in creation order, parts in insertion order
+        left = [free.get(int(type_ids[gene_type[genes[k]]])) for k in ks]
+        pos = np.array([f.pop() for f in left if f], dtype=np.int64)
         if nb_machines == 1:
             key = rng.uniform(0, 1)
         elif m == 0:
@@ -72,9 +72,7 @@ def encode(machine, place, instance_parts, type_ids, gene_type, nb_machines: int
         else:
             key = rng.uniform(thresholds[m - 1] + 0.0001, thresholds[m] - 0.0001)
         array[pos + N] = key
-        values = np.linspace(0, 1, len(pos), endpoint=False)
-        for i, p in enumerate(pos):
-            array[p] = values[i]
+        array[pos] = np.linspace(0, 1, len(pos), endpoint=False)
     return array
 
 
