@@ -22,22 +22,25 @@
 //      (chromosome, machine) items of all instances by part count.
 //   2. decode_kernel       persistent CTAs of 1, 2 or 4 warps (the launch
 //      shape), one (chromosome, machine) item at a time, longest first, from
-//      a device counter.  A plate is L rows of ceil(W/32)+2 32-bit words (bit
-//      x of a row = cell x); the first S plates of an item live in shared
-//      memory, further ones in a global pool.  For each part: first-fit over
-//      plates (area filter, then the collision search), else a new plate with
-//      the best rotation at (0, L-1).  The collision search splits (rotation,
-//      32 candidate rows) chunks over the warps, skipping chunks that cannot
-//      beat the best position found so far; a lane runs the vacancy
-//      filter of one candidate top row, then the (surviving candidate,
-//      32-column word) pairs are dealt to the lanes for the exact
-//      run-dilation test, mask rows coarse to fine from the bottom: each lane
-//      walks the first runs of its pair alone, the pairs still open are
-//      finished in order by the whole warp (a lane per run, results ANDed);
-//      the first pair with a free column gives the bottom-most candidate and
-//      its leftmost x.  Results are merged with a 64-bit lexicographic key
-//      (newLen, -y, x, rotation) by atomicMin in shared memory, which is the
-//      reference's rotation rule (binClassNew.py:101-117) — see key_of().
+//      a device counter.  A plate is a grid of L rows of ceil(W/32)+2 32-bit
+//      words (bit x of a row = cell x) and the coarse data derived from it
+//      (erosion planes and longest free runs of blocks of rows, coarse_ok());
+//      each CTA has a few plates of its own, further ones come from a global
+//      pool and stay with the CTA for its later items.  For each part:
+//      first-fit over plates (area filter, then the collision search), else a
+//      new plate with the best rotation at (0, L-1).  The collision search
+//      splits (rotation, 32 candidate rows) chunks over the warps, skipping
+//      chunks that cannot beat the best position found so far; a lane runs the
+//      vacancy filter of one candidate top row, then the (surviving candidate,
+//      64 columns) pairs are dealt to the lanes, bottom rows first: each lane
+//      tests its pair against the planes, groups of lanes test the first
+//      pieces of the runs of what is left open, and the pairs still open are
+//      finished in order by the whole warp, mask rows coarse to fine from the
+//      bottom; the first pair with a free column gives the bottom-most
+//      candidate and its leftmost x.  Results are merged with a 64-bit
+//      lexicographic key (newLen, -y, x, rotation) by atomicMin in shared
+//      memory, which is the reference's rotation rule
+//      (binClassNew.py:101-117) — see key_of().
 //   3. reduce_kernel       max over machines, 1e16 for infeasible chromosomes.
 
 #include <cuda_runtime.h>
@@ -74,16 +77,25 @@ constexpr int kDefaultTaskMax = 8192;
 // (2- and 1-warp shapes) draining SMs costs 2-7 %, so it is off there.
 constexpr int kCritItems = 16;
 constexpr int kCritSlots = 1024;  // per-SM marks, indexed by %smid
+// The coarse test's erosion planes: runs of 4, 8, 16 and 32 columns (see coarse_ok()).
+constexpr int kPlaneMin = 2;
+constexpr int kPlaneMax = 5;
 constexpr int kMaxTaskMax = 32 * 256;  // 32 candidates x the output words of the widest plate
 constexpr unsigned long long kKeyNone = ~0ull;
 constexpr unsigned kFull = 0xFFFFFFFFu;
 
 struct RotDev {
   int h, w, mw;      // rows, columns, 32-bit words per mask row
-  int vt;            // first entry in vtest[]: h (row << 16 | longest run of the row), collision-test order
   int trun, ntrun;   // runs of ones of all rows in test order: truns[trun .. trun + ntrun)
+  int tseg, ntseg;   // the same runs in pieces of at most 32 columns: tsegs[tseg .. tseg + ntseg)
   int mask_base;     // first word in maskbits[] (h * mw words)
-  int imax, dmax;    // row with the longest run of ones and that length
+};
+
+// The coarse test of one rotation at one alignment (its entries in centry[]
+// and cfilter[]); see coarse_ok() and coarse_and().
+struct CoarseIdx {
+  int e, ne;  // centry[e .. e + ne): cores as reads of two erosion-plane windows, ne even (the last one repeated)
+  int f, nf;  // cfilter[f .. f + nf): (block row << 16 | core length), nf a multiple of kVacIlp (padded with 0)
 };
 
 // The rotations of one part type that fit one machine's plate
@@ -103,6 +115,7 @@ static_assert(sizeof(RotList) == 20, "RotList layout");
 
 struct MachDev {
   int L, W, NW, RS;  // plate rows, columns, words per row, row stride (NW + 2 zero pad words)
+  int NB, PS;        // blocks of rows, words of one erosion plane (NB * RS)
   double area;       // MachineData.bin_area
   double setup;      // MachineData.setup_time
 };
@@ -134,12 +147,17 @@ struct Tables {
   const int32_t* nrot;
   const int32_t* best_rot;
   const RotDev* rot;        // [absolute type * 4 + rotation]
-  const uint32_t* vtest;
+  const CoarseIdx* cidx;    // [rotation, indexed like rot][offset of the top row in a block]
+  const uint2* centry;      // (first column | second window's offset << 16, block row | plane << 16)
+  const uint32_t* cfilter;
   const uint2* truns;       // (start | length << 16, row) per run of ones
+  const uint2* tsegs;       // the same, lengths at most 32
   const uint32_t* maskbits;
   const uint8_t* newbin_ok;
   const uint8_t* fits;
   const RotList* rl;        // [(type, machine)], indexed like fits
+  int bsh;                  // a block of the coarse test has 2^bsh rows
+  int n_planes;             // erosion plane i holds the starts of free runs of 2^(kPlaneMin + i) columns
 };
 
 // One instance's slice of a launch.
@@ -171,9 +189,12 @@ struct Run {
   int crit_items;      // items at the head of the queue that mark their SM (0 = off)
   unsigned long long* counters;
   BinScal* binscal;  // Nmax per resident CTA
-  uint32_t* pool;
+  uint32_t* pool;    // grids of the plates that are not in shared memory, grid_words each
+  uint32_t* cpool;   // their erosion planes and block vacancies, coarse_words each
   long long pool_bins;
-  int S, slot_words, slot_vac_off;
+  uint32_t* own;     // S plates per resident CTA, grid and planes
+  int S, smem_grids; // plates per item that are the CTA's own; whether their grids are in shared memory instead
+  int grid_words, coarse_words, vac_off;
   int task_max;  // most (survivor, word) pairs of a chunk dealt across lanes
   InstRun r[kMaxInst];
 };
@@ -208,9 +229,13 @@ __device__ __forceinline__ int machine_of(float mv, const double* thr, int M, in
 // W are shared and newLen * W are distinct integers <= 2^26, so the float64
 // quotients are strictly ordered by newLen: max density == min newLen.  Ties
 // go to the larger bottom row y, then the smaller x, then the first rotation.
-__device__ __forceinline__ unsigned long long key_of(int newlen, int y, int x, int r) {
-  return ((unsigned long long)newlen << 28) | ((unsigned long long)(kMaxSide - y) << 15) |
-         ((unsigned long long)x << 2) | (unsigned long long)r;
+// The row's part (newLen, y) fills the upper word, so rows compare as 32-bit values.
+__device__ __forceinline__ unsigned row_key(int newlen, int y) {
+  return ((unsigned)newlen << 13) | (unsigned)(kMaxSide - y);
+}
+
+__device__ __forceinline__ unsigned long long key_of(unsigned row, int x, int r) {
+  return ((unsigned long long)row << 32) | ((unsigned)x << 2) | (unsigned)r;
 }
 
 // bits [p, p + 32) of a row (p >= 0; reads words p>>5 and p>>5 + 1)
@@ -255,42 +280,119 @@ __device__ __forceinline__ uint32_t blocked(const uint32_t* row, int p0, int d) 
   return res;
 }
 
-constexpr int kTestIlp = 2;  // independent run dilations per step of the exact test
-constexpr int kVacIlp = 4;   // vacancy rows compared per step of the filter
-// Runs a lane walks alone before the pairs still open share the warp: a
-// sixth of the rotation's runs, between 8 and 20 (measured best on the
-// 50- to 400-part workloads).
-__device__ __forceinline__ int solo_runs(int n_runs) { return min(n_runs, min(20, max(8, n_runs / 6))); }
+// blocked() for a run of at most 32 cells and the 64 placements from p0, in
+// straight-line code (lanes with runs of different lengths stay together).
+// Reads words p0>>5 .. p0>>5 + 3, the last one only inside the row of RS words.
+__device__ __forceinline__ uint2 blocked64(const uint32_t* row, int p0, int d, int RS) {
+  const int wi = p0 >> 5;
+  const uint32_t w0 = row[wi], w1 = row[wi + 1], w2 = row[wi + 2], w3 = wi + 3 < RS ? row[wi + 3] : 0u;
+  uint32_t a = __funnelshift_r(w0, w1, p0), b = __funnelshift_r(w1, w2, p0), c = __funnelshift_r(w2, w3, p0);
+#pragma unroll
+  for (int s = 1; s < 32; s <<= 1) {
+    if (d >= 2 * s) {  // after a step bit j = OR of 2s bits from j
+      a |= __funnelshift_r(a, b, s);
+      b |= __funnelshift_r(b, c, s);
+      c |= c >> s;
+    }
+  }
+  const int rest = d - (1 << (31 - __clz(d)));  // 0 .. 15
+  return make_uint2(a | __funnelshift_r(a, b, rest), b | __funnelshift_r(b, c, rest));
+}
 
-// Necessary condition for the rotation to fit with its top row at ty: the
-// plate rows it covers have free runs at least as long as the mask rows'
-// longest runs (numba_utils.py:50-94).  The first kVacRows rows of the
-// collision-test order (widest row, then coarse to fine from the bottom)
-// are checked, kVacIlp per step so their loads overlap: a candidate
-// that fails the filter fails within them almost always, and one that slips
-// through is rejected by the exact test (24 rows measured 1 % faster than
-// 32 on the 100- to 400-part workloads, 16 rows up to 3.5 % slower).
-constexpr int kVacRows = 24;
-__device__ __forceinline__ bool vacancy_ok(const uint16_t* vac, int ty, const RotDev& rd,
-                                           const uint32_t* vtest) {
-  const uint32_t* v = vtest + rd.vt;
-  const uint16_t* row = vac + ty;
-  const int h = min(rd.h, kVacRows);
-  int i = 0;
-  for (; i + kVacIlp <= h; i += kVacIlp) {
+constexpr int kTestIlp = 2;   // independent run dilations per step of the exact test
+constexpr int kVacIlp = 2;    // block vacancies compared per step of the filter
+constexpr int kGroupOpen = 3;  // pairs open after the coarse test from which groups of lanes first test
+constexpr int kGroupSegs = 4;  // this many pieces of each
+
+// Where one open plate lives.
+struct PlateRef {
+  uint32_t* grid;    // L rows of RS words
+  uint32_t* planes;  // n_planes x NB rows of RS words
+  uint16_t* vac;     // NB longest free runs
+};
+
+// Plate b of this CTA's item: the first S in places of the CTA's own (their
+// grids in shared memory if asked for), the others in the pools.
+__device__ __forceinline__ PlateRef plate_ref(const Run& run, uint32_t* smem, int b, int pool) {
+  PlateRef pr;
+  if (b < run.S) {
+    uint32_t* own = run.own + ((size_t)blockIdx.x * run.S + b) * (run.grid_words + run.coarse_words);
+    pr.grid = run.smem_grids ? smem + (size_t)b * run.grid_words : own;
+    pr.planes = own + run.grid_words;
+  } else {
+    pr.grid = run.pool + (size_t)pool * run.grid_words;
+    pr.planes = run.cpool + (size_t)pool * run.coarse_words;
+  }
+  pr.vac = reinterpret_cast<uint16_t*>(pr.planes + run.vac_off);
+  return pr;
+}
+
+// Coarse test.  The plate also keeps, for every block of 2^bsh rows, which
+// columns are free in all of them, as erosion planes (plane i: columns at
+// which 2^(kPlaneMin + i) such columns start), and the longest run of them.
+// A rotation whose top row sits at a given offset in its block covers whole
+// blocks with 2^bsh of its rows each; the columns that all of them occupy
+// (the block's core) must be free in the plate's block.  That is a necessary
+// condition, cheap to test (a block stands for all its rows, a core for one
+// window of two plane reads instead of a dilation per row), and it rejects
+// most blocked positions before the exact test: of the (row, 32-column word)
+// pairs that pass the filter at P100M4, one in ten stays open.  What bounds the
+// kernel is integer issue on chip, so the instructions of a rejected position
+// are what counts: before, lanes walked the runs of its rows, some fifty
+// instructions for each run and 32 columns.  One launch before / now: P100M4 1.54 / 1.08 ms (500 rows) and 8.25 / 5.8 ms (4,000),
+// P200M6 3.94 / 2.58 ms (1,000), P400M8 35.9 / 19.8 ms (1,024), P50M2 0.404 /
+// 0.307 ms (1 row) and 0.523 / 0.392 ms (100), 64 uneven instances x 256
+// 29.5 / 21.1 ms.
+//
+// The filter: every block has a free run as long as the core it must take.
+__device__ __forceinline__ bool coarse_ok(const Tables& tb, const uint16_t* vac, int ty, int rot) {
+  const CoarseIdx ci = tb.cidx[(rot << tb.bsh) + (ty & ((1 << tb.bsh) - 1))];
+  const uint32_t* f = tb.cfilter + ci.f;
+  const uint16_t* v = vac + (ty >> tb.bsh);
+  for (int i = 0; i < ci.nf; i += kVacIlp) {
     bool bad = false;
 #pragma unroll
     for (int u = 0; u < kVacIlp; ++u) {
-      const uint32_t e = __ldg(v + i + u);
-      bad |= row[e >> 16] < (e & 0xFFFFu);
+      const uint32_t e = __ldg(f + i + u);
+      bad |= v[e >> 16] < (e & 0xFFFFu);
     }
     if (bad) return false;
   }
-  for (; i < h; ++i) {
-    const uint32_t e = __ldg(v + i);
-    if (row[e >> 16] < (e & 0xFFFFu)) return false;
-  }
   return true;
+}
+
+// Columns base .. base + 63 at which one core is free: its run is the union of
+// two windows of the plane's length (the entry's plane is the longest that
+// fits; longer cores are several entries).
+__device__ __forceinline__ uint2 coarse_window(const uint32_t* pl, const MachDev& md, int base, uint2 e) {
+  const uint32_t* row = pl + (e.y & 0xFFFFu) * md.RS + (e.y >> 16) * md.PS;
+  const int p = base + (int)(e.x & 0xFFFFu), q = p + (int)(e.x >> 16);
+  const uint32_t *u = row + (p >> 5), *v = row + (q >> 5);
+  const uint32_t u1 = u[1], v1 = v[1];
+  return make_uint2(__funnelshift_r(u[0], u1, p) & __funnelshift_r(v[0], v1, q),
+                    __funnelshift_r(u1, u[2], p) & __funnelshift_r(v1, v[2], q));
+}
+
+// The bits of F at which every core of rotation rot (index into tb.rot) is free, two cores per step.
+__device__ __forceinline__ uint2 coarse_and(const Tables& tb, const uint32_t* planes, const MachDev& md, int ty, int base,
+                                            uint2 F, int rot) {
+  const CoarseIdx ci = tb.cidx[(rot << tb.bsh) + (ty & ((1 << tb.bsh) - 1))];
+  const uint2* c = tb.centry + ci.e;
+  const uint32_t* pl = planes + (ty >> tb.bsh) * md.RS;
+  for (int q = 0; q < ci.ne && (F.x | F.y); q += 2) {
+    const uint2 e0 = __ldg(c + q), e1 = __ldg(c + q + 1);
+    const uint2 a = coarse_window(pl, md, base, e0), b = coarse_window(pl, md, base, e1);
+    F.x &= a.x & b.x;
+    F.y &= a.y & b.y;
+  }
+  return F;
+}
+
+// The valid candidate columns among base .. base + 63, for nx candidates in all.
+__device__ __forceinline__ uint2 first_open(int nx, int base) {
+  const int n = nx - base;
+  return make_uint2(n >= 32 ? kFull : n > 0 ? (1u << n) - 1u : 0u,
+                    n >= 64 ? kFull : n > 32 ? (1u << (n - 32)) - 1u : 0u);
 }
 
 // The bits of F (candidate columns base .. base + 31) at which the rotation
@@ -321,15 +423,16 @@ __device__ __forceinline__ uint32_t word_free(const uint32_t* g0, int RS, int ba
 
 // Leftmost x at which the rotation fits with its top row at ty, or -1
 // (output words of 32 candidate columns tried left to right).
-__device__ __forceinline__ int first_free_x(const uint32_t* grid, int RS, int W, int ty, const RotDev& rd,
-                                            const uint2* truns) {
-  const int nx = W - rd.w + 1;
-  const int nwo = (nx + 31) >> 5;
-  const uint32_t* g0 = grid + (size_t)ty * RS;
-  for (int k = 0; k < nwo; ++k) {
-    const uint32_t F0 = (k == nwo - 1 && (nx & 31)) ? ((1u << (nx & 31)) - 1u) : 0xFFFFFFFFu;
-    const uint32_t F = word_free(g0, RS, k << 5, F0, rd, truns);
-    if (F) return (k << 5) + __ffs(F) - 1;
+__device__ __forceinline__ int first_free_x(const Tables& tb, const PlateRef& pr, const MachDev& md, int ty, int rot,
+                                            const RotDev& rd) {
+  const int nx = md.W - rd.w + 1;
+  const uint32_t* g0 = pr.grid + (size_t)ty * md.RS;
+  for (int base = 0; base < nx; base += 64) {
+    const uint2 F = coarse_and(tb, pr.planes, md, ty, base, first_open(nx, base), rot);
+    const uint32_t lo = F.x ? word_free(g0, md.RS, base, F.x, rd, tb.truns) : 0u;
+    if (lo) return base + __ffs(lo) - 1;
+    const uint32_t hi = F.y ? word_free(g0, md.RS, base + 32, F.y, rd, tb.truns) : 0u;
+    if (hi) return base + 32 + __ffs(hi) - 1;
   }
   return -1;
 }
@@ -354,13 +457,20 @@ __device__ __forceinline__ int longest_ones(uint32_t x) {
   return n;
 }
 
-// longest run of empty cells in a plate row (numba_utils.py:160-188)
-__device__ int max_zero_run(const uint32_t* row, int W, int NW) {
+// free columns of a block of plate rows in word w: bit set = no row occupies it (columns past W count as occupied)
+__device__ __forceinline__ uint32_t block_free(const uint32_t* row, const MachDev& md, int rows, int w) {
+  uint32_t v = 0u;
+  for (int i = 0; i < rows; ++i) v |= row[(size_t)i * md.RS + w];
+  const int valid = md.W - 32 * w;
+  if (valid < 32) v |= 0xFFFFFFFFu << valid;
+  return ~v;
+}
+
+// longest run of free columns of a block of plate rows (plates wider than 1024 columns; one thread)
+__device__ int max_free_run(const uint32_t* row, const MachDev& md, int rows) {
   int run = 0, best = 0;
-  for (int w = 0; w < NW; ++w) {
-    uint32_t v = row[w];
-    const int valid = W - 32 * w;
-    if (valid < 32) v |= 0xFFFFFFFFu << valid;
+  for (int w = 0; w < md.NW; ++w) {
+    const uint32_t v = ~block_free(row, md, rows, w);
     if (v == 0u) {
       run += 32;
       continue;
@@ -379,14 +489,13 @@ __device__ __forceinline__ void raise_status(int32_t* status, int code) {
   atomicCAS(status, 0, code);
 }
 
-// The window a (candidate, output word) pair of the exact test reads: plate
-// rows row0 .. row0 + h - 1 and, in each, the words that the dilations of the
-// mask's runs touch for the 32 columns base .. base + 31 — at most word
-// ((base + w + 31) >> 5) + 1 (a run starts at s >= 0 with s + d <= w, a table
-// invariant of the rotation's run list).  Checked once per pair, so the runs
-// inside need no check of their own.
-__device__ __forceinline__ bool pair_in_plate(int row0, int base, const RotDev& rd, const MachDev& md) {
-  return row0 >= 0 && row0 + rd.h <= md.L && base >= 0 && ((base + rd.w + 31) >> 5) + 1 < md.RS;
+// The window that a (candidate, 64-column word) pair of the tests reads: plate
+// rows row0 .. row0 + h - 1 and, in each, at most word ((base + w - 1) >> 5) + 2
+// (a run starts at s >= 0 with s + d <= w, a table invariant; the exact test
+// checks the word after that one itself).  Checked once per pair, so the
+// cores and runs inside need no check of their own.
+__device__ __forceinline__ bool pair_in_plate(int row0, int base, int h, int w, const MachDev& md) {
+  return row0 >= 0 && row0 + h <= md.L && base >= 0 && base + w <= md.W;
 }
 
 // Instance of a launch row / item: the last instance starting at or before v
@@ -518,8 +627,9 @@ struct SearchShared {
   unsigned long long best;
   int chunk, total, nr;
   int rlist[4];
-  int rh[4];      // heights of the rotations in rlist
-  RotDev rd[4];   // their descriptors, read by every chunk
+  RotDev rd[4];      // their descriptors, read by every chunk
+  int nw[4];         // 64-column words of their candidates in a row
+  unsigned inv[4];   // ceil(2^32 / nw)
   unsigned char surv[kWarps][32];  // per warp: lanes whose candidate passed the vacancy filter
 };
 
@@ -531,7 +641,7 @@ struct SearchShared {
 // all threads of the CTA; contains __syncthreads.
 template <int kWarps>
 __device__ __forceinline__ unsigned long long search_plate(const Tables& tb, const MachDev& md,
-                                                           const uint32_t* grid, const uint16_t* vac, int enc,
+                                                           const PlateRef& pr, int enc,
                                                            int t, const RotList* rlp, int task_max, int32_t* status,
                                                            SearchShared<kWarps>& sh,
                                                            unsigned long long& c_tests,
@@ -540,17 +650,16 @@ __device__ __forceinline__ unsigned long long search_plate(const Tables& tb, con
   const int tid = threadIdx.x, lane = tid & 31;
   if (tid < 4) {  // one thread per rotation: the list was built at problem creation
     const int nr0 = rlp->nr;
-    // With fewer than four warps a level's chunks are taken one after another:
-    // the shortest rotation first has the smallest best-case key and prunes
-    // the others sooner (measured 4.5 % off the 2-warp P200M6 launch; with
-    // four warps every rotation of a level starts at once and the order only
-    // cost time).
+    // The shortest rotation first has the smallest best-case key and prunes
+    // the others sooner (measured 2-4 % off in every launch shape).
     if (tid < nr0) {
-      const int r = blockDim.x < 128 ? rlp->rs[tid] : rlp->r[tid];
+      const int r = rlp->rs[tid];
       const RotDev rd = tb.rot[t * 4 + r];
+      const int nw = (md.W - rd.w + 64) >> 6;
       sh.rlist[tid] = r;
-      sh.rh[tid] = rd.h;
       sh.rd[tid] = rd;
+      sh.nw[tid] = nw;
+      sh.inv[tid] = nw > 1 ? 0xFFFFFFFFu / (unsigned)nw + 1u : 0u;
     }
     if (tid == 0) {
       sh.nr = nr0;
@@ -563,153 +672,143 @@ __device__ __forceinline__ unsigned long long search_plate(const Tables& tb, con
   }
   __syncthreads();
   const int nr = sh.nr, total = sh.total;
+  unsigned char* surv = sh.surv[tid >> 5];
   for (int guard = 0; guard < total; ++guard) {
     int ci = 0;
-    if (lane == 0) ci = atomicAdd(&sh.chunk, 1);
+    unsigned long long best = 0;
+    if (lane == 0) {
+      ci = atomicAdd(&sh.chunk, 1);
+      best = *(volatile unsigned long long*)&sh.best;
+    }
     ci = __shfl_sync(kFull, ci, 0);
     if (ci >= total) break;
+    best = __shfl_sync(kFull, best, 0);
     const int level = nr == 4 ? ci >> 2 : nr == 2 ? ci >> 1 : nr == 1 ? ci : ci / 3;
     const int slot = ci - level * nr;
-    const int r = sh.rlist[slot];
-    const RotDev rd = sh.rd[slot];
-    const int ty_hi = md.L - rd.h - 32 * level;
+    const int h = sh.rd[slot].h, r = sh.rlist[slot];
+    const int ty_hi = md.L - h - 32 * level;
     if (ty_hi < 0) continue;
-    unsigned long long cur = 0;
-    if (lane == 0) cur = *(volatile unsigned long long*)&sh.best;
-    cur = __shfl_sync(kFull, cur, 0);
-    if (key_of(max(enc, md.L - ty_hi), ty_hi + rd.h - 1, 0, r) >= cur) {
+    if (key_of(row_key(max(enc, md.L - ty_hi), ty_hi + h - 1), 0, r) >= best) {
       // The best key a chunk can give only grows with its level, and the best
       // found only shrinks: when no rotation can beat it at this level, no
       // later chunk (same level or higher) can, and the warp is done.
       bool beat = false;
       for (int j = 0; j < nr; ++j) {
-        const int tyj = md.L - sh.rh[j] - 32 * level;
-        beat |= tyj >= 0 && key_of(max(enc, md.L - tyj), tyj + sh.rh[j] - 1, 0, sh.rlist[j]) < cur;
+        const int hj = sh.rd[j].h, tyj = md.L - hj - 32 * level;
+        beat |= tyj >= 0 && key_of(row_key(max(enc, md.L - tyj), tyj + hj - 1), 0, sh.rlist[j]) < best;
       }
       if (!beat) break;
       continue;
     }
-    const int ty = ty_hi - lane;
     if (lane == 0) ++c_chunks;
-    // Vacancy filter one candidate per lane.  Then, when there are few enough
-    // (survivor, output word) pairs, they are dealt to the lanes in rounds of
-    // 32, bottom-most survivor and leftmost word first, so lanes whose
-    // candidate failed the filter take part in the exact test of the others;
-    // in a round each lane first walks a few runs of its pair alone, then the
-    // pairs still open are finished by the whole warp in order, and the first
-    // pair with a free column is the bottom-most candidate's leftmost x.
+    // Vacancy filter, one candidate row per lane.  Then, when there are few
+    // enough (surviving row, 64 candidate columns) pairs, they are dealt to the
+    // lanes in rounds of 32, bottom-most row and leftmost columns first:
+    //   1. each lane tests its pair's cores against the erosion planes;
+    //   2. where that leaves several pairs open, groups of lanes test the first
+    //      pieces of their runs;
+    //   3. the pairs still open are finished in order by the whole warp: every
+    //      lane walks every 32nd piece of the mask's runs, the lanes' blocked
+    //      columns are ORed after each step.  The first pair that stays free is
+    //      the bottom-most candidate's leftmost x, and the chunk is done.
     // Otherwise each lane tests its own candidate's words left to right.
-    const bool pass = ty >= 0 && vacancy_ok(vac, ty, rd, tb.vtest);
+    const int ty = ty_hi - lane, rot = t * 4 + r, nx = md.W - sh.rd[slot].w + 1;
+    const bool pass = ty >= 0 && coarse_ok(tb, pr.vac, ty, rot);
     const unsigned S = __ballot_sync(kFull, pass);
     if (!S) continue;
-    const int nx = md.W - rd.w + 1, nwo = (nx + 31) >> 5;
-    const int ntask = __popc(S) * nwo;
-    if (ntask <= task_max) {
-      unsigned char* surv = sh.surv[tid >> 5];
-      if (pass) surv[__popc(S & ((1u << lane) - 1u))] = (unsigned char)lane;
-      __syncwarp();
-      const uint32_t Flast = (nx & 31) ? ((1u << (nx & 31)) - 1u) : kFull;
-      const uint2* runs = tb.truns + rd.trun;
-      const int n_runs = rd.ntrun, qsolo = solo_runs(n_runs);
-      for (int t0 = 0; t0 < ntask; t0 += 32) {
-        {  // the round's first pair has the smallest key left in the chunk: stop when it cannot win
-          unsigned long long cur = 0;
-          if (lane == 0) cur = *(volatile unsigned long long*)&sh.best;
-          cur = __shfl_sync(kFull, cur, 0);
-          const int si0 = t0 / nwo, k0 = t0 - si0 * nwo;
-          const int ty0 = ty_hi - surv[si0];
-          if (key_of(max(enc, md.L - ty0), ty0 + rd.h - 1, k0 << 5, r) >= cur) break;
-        }
-        // Solo phase: each lane walks the first runs of its own pair, two per
-        // step; most blocked words close within them.
-        const int t = t0 + lane;
-        uint32_t F = 0u;
-        int k = 0, sl = 0, q = 0;
-        if (t < ntask) {
-          const int si = t / nwo;
-          k = t - si * nwo;
-          sl = surv[si];
-          F = k == nwo - 1 ? Flast : kFull;
-          const int row0 = ty_hi - sl, base = k << 5;
-          if (!pair_in_plate(row0, base, rd, md)) {  // never on consistent tables: skip the pair, flag the launch
-            raise_status(status, BRKGA_ERR_INTERNAL);
-            F = 0u;
-          }
-          const uint32_t* g0 = grid + (size_t)row0 * md.RS;
-          for (; q < qsolo && F; q += 2) {
-            const uint2 e0 = __ldg(runs + q);
-            uint32_t bl = blocked(g0 + (int)e0.y * md.RS, base + (int)(e0.x & 0xFFFFu), (int)(e0.x >> 16));
-            if (q + 1 < qsolo) {
-              const uint2 e1 = __ldg(runs + q + 1);
-              bl |= blocked(g0 + (int)e1.y * md.RS, base + (int)(e1.x & 0xFFFFu), (int)(e1.x >> 16));
-            }
-            F &= ~bl;
-          }
-          q = min(q, qsolo);
-        }
-        // Shared phase: a pair with runs left and columns open is walked by the
-        // whole warp, in task order, up to the first pair already proven free
-        // (pairs after it cannot win): every lane takes every 32nd remaining
-        // run on its own, then the lanes AND their open columns.  The first
-        // pair that stays free is the bottom-most candidate's leftmost x.
-        const unsigned open = __ballot_sync(kFull, F != 0u && q < n_runs);
-        const unsigned done_free = __ballot_sync(kFull, F != 0u && q >= n_runs);
-        unsigned rem = open & (done_free ? ((done_free & (0u - done_free)) - 1u) : kFull);
-        int win = done_free ? __ffs(done_free) - 1 : -1;
-        uint32_t Fw = __shfl_sync(kFull, F, win < 0 ? 0 : win);
-        while (rem) {
-          const int l = __ffs(rem) - 1;
-          rem &= rem - 1u;
-          uint32_t Fp = __shfl_sync(kFull, F, l);
-          const int ql = __shfl_sync(kFull, q, l);
-          const int kl = __shfl_sync(kFull, k, l);
-          const int sll = __shfl_sync(kFull, sl, l);
-          const int row0 = ty_hi - sll, base = kl << 5;
-          {  // pairs come in key order: stop when this one cannot beat the best found
-            unsigned long long cur = 0;
-            if (lane == 0) cur = *(volatile unsigned long long*)&sh.best;
-            cur = __shfl_sync(kFull, cur, 0);
-            if (key_of(max(enc, md.L - row0), row0 + rd.h - 1, base + __ffs(Fp) - 1, r) >= cur) {
-              win = -1;
-              break;
-            }
-          }
-          if (!pair_in_plate(row0, base, rd, md)) {  // warp-uniform: the pair's values came from shuffles
-            if (lane == 0) raise_status(status, BRKGA_ERR_INTERNAL);
-            continue;
-          }
-          const uint32_t* g0 = grid + (size_t)row0 * md.RS;
-          for (int qq = ql + lane; qq < n_runs && Fp; qq += 32) {
-            const uint2 e = __ldg(runs + qq);
-            Fp &= ~blocked(g0 + (int)e.y * md.RS, base + (int)(e.x & 0xFFFFu), (int)(e.x >> 16));
-          }
-          for (int o = 1; o < 32; o <<= 1) Fp &= __shfl_xor_sync(kFull, Fp, o);
-          if (Fp) {
-            win = l;
-            Fw = Fp;
-            break;
-          }
-        }
-        if (win >= 0) {
-          const int kb = __shfl_sync(kFull, k, win);
-          const int slb = __shfl_sync(kFull, sl, win);
-          if (lane == 0) {
-            const int tyb = ty_hi - slb;
-            atomicMin(&sh.best, key_of(max(enc, md.L - tyb), tyb + rd.h - 1, (kb << 5) + __ffs(Fw) - 1, r));
-          }
-          break;
-        }
-      }
-      __syncwarp();
-    } else {
-      const int x = pass ? first_free_x(grid, md.RS, md.W, ty, rd, tb.truns) : -1;
+    const int nw = sh.nw[slot], ntask = __popc(S) * nw;
+    if (ntask > task_max) {
+      const int x = pass ? first_free_x(tb, pr, md, ty, rot, sh.rd[slot]) : -1;
       const unsigned fm = __ballot_sync(kFull, x >= 0);
       if (fm) {
         const int l = __ffs(fm) - 1;
         const int xb = __shfl_sync(kFull, x, l);
-        if (lane == 0) {
-          const int tyb = ty_hi - l;
-          atomicMin(&sh.best, key_of(max(enc, md.L - tyb), tyb + rd.h - 1, xb, r));
+        if (lane == 0)
+          atomicMin(&sh.best, key_of(row_key(max(enc, md.L - (ty_hi - l)), ty_hi - l + h - 1), xb, r));
+      }
+      continue;
+    }
+    __syncwarp();  // the last chunk's list is read
+    if (pass) surv[__popc(S & ((1u << lane) - 1u))] = (unsigned char)lane;
+    __syncwarp();
+    const unsigned inv = sh.inv[slot];
+    const uint2* segs = tb.tsegs + sh.rd[slot].tseg;
+    const int nseg = sh.rd[slot].ntseg;
+    bool won = false;
+    for (int t0 = 0; t0 < ntask && !won; t0 += 32) {
+      // ---- the round's first pair has the smallest key left in the chunk: stop when it cannot win
+      if (lane == 0) best = *(volatile unsigned long long*)&sh.best;
+      best = __shfl_sync(kFull, best, 0);
+      const int ti = t0 + lane, si = nw > 1 ? (int)__umulhi((unsigned)ti, inv) : ti;
+      const int base = (ti - si * nw) << 6, row0 = ti < ntask ? ty_hi - surv[si] : 0;
+      const unsigned long long low = key_of(row_key(max(enc, md.L - row0), row0 + h - 1), base, r);
+      if (__shfl_sync(kFull, low, 0) >= best) break;
+      // ---- coarse test of one pair per lane
+      uint2 F = make_uint2(0u, 0u);
+      if (ti < ntask) {
+        if (pair_in_plate(row0, base, h, md.W - nx + 1, md)) {
+          F = coarse_and(tb, pr.planes, md, row0, base, first_open(nx, base), rot);
+        } else {  // never on consistent tables: skip the pair, flag the launch
+          raise_status(status, BRKGA_ERR_INTERNAL);
+        }
+      }
+      unsigned open = __ballot_sync(kFull, (F.x | F.y) != 0u);
+      const int n_open = __popc(open), pk = row0 << 13 | base;
+      int q0 = 0;
+      // ---- several pairs open: 32 / 2^lg of them at once, 2^lg lanes each
+      if (n_open >= kGroupOpen) {
+        const int lg = n_open <= 4 ? 3 : n_open <= 8 ? 2 : n_open <= 16 ? 1 : 0;
+        unsigned m = open;
+        for (int k = 0; k < (32 >> lg) - 1; ++k)
+          if (k < lane >> lg) m &= m - 1u;  // drop the pairs of the groups below
+        const int src = m ? __ffs(m) - 1 : 0;
+        const int pl = __shfl_sync(kFull, pk, src);
+        uint32_t lo = __shfl_sync(kFull, F.x, src), hi = __shfl_sync(kFull, F.y, src);
+        if (!m) lo = hi = 0u;
+        const int basel = pl & 0x1FFF, n = min(max(kGroupSegs, 1 << lg), nseg);
+        const uint32_t* g0 = pr.grid + (size_t)(pl >> 13) * md.RS;
+        for (int q = lane & ((1 << lg) - 1); q < n && (lo | hi); q += 1 << lg) {
+          const uint2 e = __ldg(segs + q);
+          const uint2 b = blocked64(g0 + (size_t)e.y * md.RS, basel + (int)(e.x & 0xFFFFu), (int)(e.x >> 16), md.RS);
+          lo &= ~b.x;
+          hi &= ~b.y;
+        }
+        __syncwarp();
+        for (int o = 1; o < 1 << lg; o <<= 1) {
+          lo &= __shfl_xor_sync(kFull, lo, o);
+          hi &= __shfl_xor_sync(kFull, hi, o);
+        }
+        const int from = __popc(open & ((1u << lane) - 1u)) << lg;  // this lane's pair was the group's at `from`
+        F.x &= __shfl_sync(kFull, lo, from & 31);
+        F.y &= __shfl_sync(kFull, hi, from & 31);
+        open &= __ballot_sync(kFull, (F.x | F.y) != 0u);
+        q0 = max(kGroupSegs, 1 << lg);
+      }
+      // ---- exact test of the open pairs in order
+      while (open) {
+        const int l = __ffs(open) - 1;
+        open &= open - 1u;
+        const int pl = __shfl_sync(kFull, pk, l);
+        uint32_t lo = __shfl_sync(kFull, F.x, l), hi = __shfl_sync(kFull, F.y, l);
+        const int basel = pl & 0x1FFF, rowl = pl >> 13;
+        const unsigned rk = row_key(max(enc, md.L - rowl), rowl + h - 1);
+        if (key_of(rk, basel, r) >= best) break;
+        const uint32_t* g0 = pr.grid + (size_t)rowl * md.RS;
+        for (int q = q0; q < nseg && (lo | hi); q += 32) {
+          uint32_t bx = 0u, by = 0u;
+          if (q + lane < nseg) {
+            const uint2 e = __ldg(segs + q + lane);
+            const uint2 b = blocked64(g0 + (size_t)e.y * md.RS, basel + (int)(e.x & 0xFFFFu), (int)(e.x >> 16), md.RS);
+            bx = b.x;
+            by = b.y;
+          }
+          lo &= ~__reduce_or_sync(kFull, bx);
+          hi &= ~__reduce_or_sync(kFull, by);
+        }
+        if (lo | hi) {
+          if (lane == 0) atomicMin(&sh.best, key_of(rk, basel + (lo ? __ffs(lo) - 1 : 31 + __ffs(hi)), r));
+          won = true;
+          break;
         }
       }
     }
@@ -718,22 +817,68 @@ __device__ __forceinline__ unsigned long long search_plate(const Tables& tb, con
   return sh.best;
 }
 
+// The erosion planes and vacancies of blocks b0 .. b1 of a plate, from its
+// rows.  A group of 8, 16 or 32 lanes takes a block, a lane one word of it (on
+// plates wider than 1024 columns a warp walks the row in steps that overlap by
+// the words an erosion reaches).  All threads of the CTA; no barrier.
+__device__ __forceinline__ void update_blocks(const Tables& tb, const MachDev& md, const PlateRef& pr, int b0, int b1) {
+  const int lane = threadIdx.x & 31;
+  const int G = md.NW <= 8 ? 8 : md.NW <= 16 ? 16 : 32, gl = lane & (G - 1);
+  const int groups = blockDim.x / G;
+  constexpr int kReach = (1 << kPlaneMax) / 32 + 1;  // words past its own that a plane word depends on
+  const int step = md.NW <= 32 ? 32 : 32 - kReach;
+  for (int bb = b0; bb <= b1; bb += groups) {
+    const int b = bb + (int)threadIdx.x / G;
+    const bool on = b <= b1;
+    const uint32_t* row = pr.grid + (size_t)(b << tb.bsh) * md.RS;
+    const int rows = min(1 << tb.bsh, md.L - (b << tb.bsh));
+    for (int w0 = 0; w0 < md.NW; w0 += step) {
+      const int w = w0 + gl;
+      const uint32_t e0 = on && w < md.NW ? block_free(row, md, rows, w) : 0u;
+      uint32_t* dst = pr.planes + (size_t)b * md.RS + w;
+      const bool put = on && w < md.NW && gl < step;
+      uint32_t e = e0;
+#pragma unroll
+      for (int k = 1; k <= kPlaneMax; ++k) {
+        if (k >= kPlaneMin + tb.n_planes) break;
+        uint32_t nx = __shfl_down_sync(kFull, e, 1, G);
+        if (gl + 1 >= G) nx = 0u;
+        e &= __funnelshift_r(e, nx, 1 << (k - 1));
+        if (k >= kPlaneMin && put) dst[(size_t)(k - kPlaneMin) * md.PS] = e;
+      }
+      if (md.NW <= 32) {
+        // longest run of set bits over the group's words: inside a word, or
+        // from a word's top bits through full words into the next one's low bits
+        const unsigned fm = __ballot_sync(kFull, e0 == kFull) >> (lane - gl);
+        const unsigned rest = ~(fm >> gl >> 1);  // bit i: lane gl + 1 + i is not full
+        const int hop = min(__ffs(rest) - 1, G - 1 - gl);  // full lanes that follow
+        const int low = e0 == kFull ? 32 : __ffs(~e0) - 1;
+        int end = __shfl_sync(kFull, low, lane - gl + min(gl + 1 + hop, G - 1));
+        if (gl + 1 + hop >= G) end = 0;
+        int run = longest_ones(e0);
+        if (e0 != kFull || gl == 0) run = max(run, (e0 == kFull ? 32 : __clz(~e0)) + 32 * hop + end);
+        for (int o = G >> 1; o; o >>= 1) run = max(run, __shfl_xor_sync(kFull, run, o, G));
+        if (on && gl == 0) pr.vac[b] = (uint16_t)run;
+      }
+    }
+    if (md.NW > 32 && on && gl == 0) pr.vac[b] = (uint16_t)max_free_run(row, md, rows);
+  }
+}
+
 // Insert rotation r of part type t (absolute) with its top row at ty and left
 // column x (binClassNew.py:155-174): OR the mask rows into the plate words,
-// recompute the vacancy of the touched rows (numba_utils.py:160-188); thread 0
-// updates the plate scalars with the part's area and times on this machine.
-// One thread per mask row does both the OR of its row and that plate row's
-// vacancy (a plate row is touched by one mask row only), so no barrier
-// separates them.  All threads of the CTA; ends with __syncthreads.
-__device__ __forceinline__ void place_part(const Tables& tb, const MachDev& md, uint32_t* grid, uint16_t* vac,
-                                           BinScal* scal, int t, int r, int x, int ty, double a, double ptv,
-                                           double pthv) {
+// then recompute the touched blocks' planes and vacancies; thread 0 updates
+// the plate scalars with the part's area and times on this machine.  Without
+// `cells` (no search of the item follows) only the scalars.
+// All threads of the CTA; ends with __syncthreads.
+__device__ __forceinline__ void place_part(const Tables& tb, const MachDev& md, const PlateRef& pr, BinScal* scal, int t,
+                                           int r, int x, int ty, double a, double ptv, double pthv, bool cells) {
   const int tid = threadIdx.x;
   const RotDev rd = tb.rot[t * 4 + r];
   const int sx = x & 31, wx = x >> 5, mw = rd.mw;
   const uint32_t* mb = tb.maskbits + rd.mask_base;
-  for (int i = tid; i < rd.h; i += blockDim.x) {
-    uint32_t* row = grid + (size_t)(ty + i) * md.RS;
+  for (int i = tid; i < rd.h && cells; i += blockDim.x) {
+    uint32_t* row = pr.grid + (size_t)(ty + i) * md.RS;
     const uint32_t* m = mb + (size_t)i * mw;
     uint32_t* dst = row + wx;
     if (mw <= 8) {  // all loads first, so their latencies overlap
@@ -762,7 +907,6 @@ __device__ __forceinline__ void place_part(const Tables& tb, const MachDev& md, 
       const uint32_t v = __funnelshift_l(prev, 0u, sx);
       if (v) dst[mw] |= v;
     }
-    vac[ty + i] = (uint16_t)max_zero_run(row, md.W, md.NW);
   }
   if (tid == 0) {
     BinScal s = *scal;
@@ -775,14 +919,29 @@ __device__ __forceinline__ void place_part(const Tables& tb, const MachDev& md, 
     *scal = s;
   }
   __syncthreads();
+  if (!cells) return;
+  update_blocks(tb, md, pr, ty >> tb.bsh, (ty + rd.h - 1) >> tb.bsh);
+  __syncthreads();
 }
 
-// Empty plate: zero words, vacancy W (binClassNew.py:18-20), fresh scalars.
-__device__ __forceinline__ void open_plate(const MachDev& md, uint32_t* grid, uint16_t* vac, BinScal* scal,
-                                           int pool_index) {
+// Empty plate: zero words, every run of columns free (binClassNew.py:18-20),
+// fresh scalars.  Without `cells` only the scalars.
+__device__ __forceinline__ void open_plate(const Tables& tb, const MachDev& md, const PlateRef& pr, BinScal* scal,
+                                           int pool_index, bool cells) {
   const int tid = threadIdx.x;
-  for (int i = tid; i < md.L * md.RS; i += blockDim.x) grid[i] = 0u;
-  for (int i = tid; i < md.L; i += blockDim.x) vac[i] = (uint16_t)md.W;
+  if (cells) {
+    for (int i = tid; i < md.L * md.RS; i += blockDim.x) pr.grid[i] = 0u;
+    const int step = (int)blockDim.x % md.RS;
+    for (int i = tid, w = tid % md.RS; i < md.PS; i += blockDim.x) {  // w: the word's place in its row
+      for (int p = 0; p < tb.n_planes; ++p) {
+        const int n = md.W - (1 << (kPlaneMin + p)) + 1 - 32 * w;  // run starts from this word on
+        pr.planes[(size_t)p * md.PS + i] = n <= 0 ? 0u : n >= 32 ? kFull : (1u << n) - 1u;
+      }
+      w += step;
+      if (w >= md.RS) w -= md.RS;
+    }
+    for (int i = tid; i < md.NB; i += blockDim.x) pr.vac[i] = (uint16_t)md.W;
+  }
   if (tid == 0) {
     BinScal z;
     z.area = 0.0;
@@ -800,7 +959,7 @@ __device__ __forceinline__ void open_plate(const MachDev& md, uint32_t* grid, ui
 __device__ __forceinline__ void decode_key(unsigned long long key, int* r, int* x, int* y) {
   *r = (int)(key & 3ull);
   *x = (int)((key >> 2) & 0x1FFFull);
-  *y = kMaxSide - (int)((key >> 15) & 0x1FFFull);
+  *y = kMaxSide - (int)((key >> 32) & 0x1FFFull);
 }
 
 // The item a CTA is decoding, set up by thread 0.
@@ -831,6 +990,7 @@ __global__ void __launch_bounds__(kThreads, kResidentWarps * 32 / kThreads)
   __shared__ SearchShared<kThreads / 32> sh2[2];
   __shared__ ItemCtx ctx;
   int sh_par = 0;
+  int owned = 0;  // pool plates this CTA holds, in bs[S .. S + owned)
   __shared__ int s_fail, s_pool;
   const int tid = threadIdx.x, lane = tid & 31;
   BinScal* bs = run.binscal + (size_t)blockIdx.x * run.Nmax;
@@ -905,13 +1065,10 @@ __global__ void __launch_bounds__(kThreads, kResidentWarps * 32 / kThreads)
       // ---- first fit over the open plates (placement.py:56-64)
       for (int b = 0; b < nb; ++b) {
         if (bs[b].area + a > md.area) continue;  // placement.py:57-59
-        const uint32_t* grid = b < run.S ? smem + (size_t)b * run.slot_words
-                                         : run.pool + (size_t)bs[b].pool * run.slot_words;
-        const uint16_t* vac = reinterpret_cast<const uint16_t*>(grid + run.slot_vac_off);
-        key = search_plate(tb, md, grid, vac, bs[b].enc, t,
+        const PlateRef pr = plate_ref(run, smem, b, bs[b].pool);
+        key = search_plate(tb, md, pr, bs[b].enc, t,
                            tb.rl + ctx.tmbase + (size_t)(t - ctx.tbase) * ctx.M + ctx.m, run.task_max, run.status,
-                           sh2[sh_par], c_tests,
-                           c_chunks, c_bytes);
+                           sh2[sh_par], c_tests, c_chunks, c_bytes);
         sh_par ^= 1;
         if (key != kKeyNone) {
           pb = b;
@@ -919,6 +1076,7 @@ __global__ void __launch_bounds__(kThreads, kResidentWarps * 32 / kThreads)
         }
       }
 
+      const bool last = k + 1 == n;  // no search follows: the plate's cells are not needed
       int r, x, ty;
       if (pb < 0) {
         // ---- new plate, best rotation at column 0, bottom row L-1 (placement.py:66-83)
@@ -929,7 +1087,8 @@ __global__ void __launch_bounds__(kThreads, kResidentWarps * 32 / kThreads)
           if (!tb.newbin_ok[ctx.tmbase + (t - ctx.tbase) * ctx.M + ctx.m]) {
             s_fail = BRKGA_ERR_NEW_BIN_UNFIT;
           } else if (nb >= run.S) {
-            const unsigned idx = atomicAdd(run.pool_ctr, 1u);
+            // a pool plate taken for an earlier item stays this CTA's
+            const unsigned idx = nb - run.S < owned ? (unsigned)bs[nb].pool : atomicAdd(run.pool_ctr, 1u);
             if ((long long)idx >= run.pool_bins) s_fail = BRKGA_ERR_CAPACITY;
             else s_pool = (int)idx;
           }
@@ -944,8 +1103,8 @@ __global__ void __launch_bounds__(kThreads, kResidentWarps * 32 / kThreads)
           break;
         }
         pb = nb++;
-        uint32_t* grid = pb < run.S ? smem + (size_t)pb * run.slot_words : run.pool + (size_t)s_pool * run.slot_words;
-        open_plate(md, grid, reinterpret_cast<uint16_t*>(grid + run.slot_vac_off), &bs[pb], s_pool);
+        owned = max(owned, nb - run.S);
+        open_plate(tb, md, plate_ref(run, smem, pb, s_pool), &bs[pb], s_pool, !last);
         if (tid == 0) ++c_bins;
         x = 0;
         ty = md.L - tb.rot[t * 4 + r].h;
@@ -956,10 +1115,8 @@ __global__ void __launch_bounds__(kThreads, kResidentWarps * 32 / kThreads)
       }
 
       // ---- insert (binClassNew.py:155-174)
-      uint32_t* grid = pb < run.S ? smem + (size_t)pb * run.slot_words : run.pool + (size_t)bs[pb].pool * run.slot_words;
       const size_t tm = (size_t)ctx.tmbase + (size_t)ctx.m * ctx.T + (t - ctx.tbase);
-      place_part(tb, md, grid, reinterpret_cast<uint16_t*>(grid + run.slot_vac_off), &bs[pb], t, r, x, ty, a,
-                 tb.pt[tm], tb.pth[tm]);
+      place_part(tb, md, plate_ref(run, smem, pb, bs[pb].pool), &bs[pb], t, r, x, ty, a, tb.pt[tm], tb.pth[tm], !last);
       if (tid == 0 && lg) lg[k] = BrkgaPlacement{gene, pb, x, ty + tb.rot[t * 4 + r].h - 1, r};
     }
     if (!failed && tid == 0) {  // placement.py:86-89
@@ -1026,7 +1183,8 @@ struct GreedyArgs {
   int32_t* status;
   BinScal* binscal;
   uint32_t* pool;
-  int slot_words, slot_vac_off;
+  uint32_t* cpool;
+  int grid_words, coarse_words, vac_off;
   const int32_t* order;
   int n;
   int32_t* out_machine;  // [n]
@@ -1042,6 +1200,11 @@ struct GreedyArgs {
 // and their number.  In shared memory as long as it fits (up to some 8,000 parts).
 size_t greedy_state_bytes(int n, int M) { return (size_t)n * 28 + (size_t)M * 20; }
 constexpr size_t kGreedyMaxSmem = 229 * 1024;
+
+__device__ __forceinline__ PlateRef greedy_plate(const GreedyArgs& g, int b) {
+  uint32_t* planes = g.cpool + (size_t)b * g.coarse_words;
+  return PlateRef{g.pool + (size_t)b * g.grid_words, planes, reinterpret_cast<uint16_t*>(planes + g.vac_off)};
+}
 
 __device__ __forceinline__ unsigned cluster_rank() {
   unsigned r;
@@ -1104,8 +1267,8 @@ __global__ void __launch_bounds__(kGreedyThreads) greedy_kernel(const __grid_con
       const MachDev md = tb.mach[m];
       unsigned long long key = kKeyNone;
       if (tb.fits[t * g.M + m]) {  // BRKGA_alg3.py:465-470
-        const uint32_t* grid = g.pool + (size_t)b * g.slot_words;
-        key = search_plate(tb, md, grid, reinterpret_cast<const uint16_t*>(grid + g.slot_vac_off), bs[b].enc, t,
+        const PlateRef pr = greedy_plate(g, b);
+        key = search_plate(tb, md, pr, bs[b].enc, t,
                            tb.rl + (size_t)t * g.M + m, kDefaultTaskMax, g.status, sh2[sh_par], c_tests, c_chunks,
                            c_bytes);
         sh_par ^= 1;
@@ -1187,11 +1350,10 @@ __global__ void __launch_bounds__(kGreedyThreads) greedy_kernel(const __grid_con
     }
     cw = cw > c.cand ? cw : c.cand;
     if ((unsigned)b % kGreedyCtas == rank) {
-      uint32_t* grid = g.pool + (size_t)b * g.slot_words;
-      uint16_t* vac = reinterpret_cast<uint16_t*>(grid + g.slot_vac_off);
-      if (fresh) open_plate(md, grid, vac, &bs[b], c.machine);
-      place_part(tb, md, grid, vac, &bs[b], t, r, x, ty, a, tb.pt[(size_t)c.machine * g.T + t],
-                 tb.pth[(size_t)c.machine * g.T + t]);
+      const PlateRef pr = greedy_plate(g, b);
+      if (fresh) open_plate(tb, md, pr, &bs[b], c.machine, true);
+      place_part(tb, md, pr, &bs[b], t, r, x, ty, a, tb.pt[(size_t)c.machine * g.T + t],
+                 tb.pth[(size_t)c.machine * g.T + t], true);
       if (tid == 0) {
         g.out_machine[k] = c.machine;
         g.out[k] = BrkgaPlacement{gene, g.plate_index[b], x, ty + tb.rot[t * 4 + r].h - 1, r};
@@ -1281,7 +1443,7 @@ __global__ void __launch_bounds__(corr::kThreads, 1) chunk_free_i8_kernel(const 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 struct Layout {
-  size_t off_ctr, off_crit, off_seq, off_cnt, off_inf, off_ord, off_mk, off_bins, off_pool, total;
+  size_t off_ctr, off_crit, off_seq, off_cnt, off_inf, off_ord, off_mk, off_bins, off_pool, end_pool, off_cpool, total;
 };
 
 // Sizes of one launch: chromosome rows, (chromosome, machine) items, part-order entries.
@@ -1293,8 +1455,8 @@ struct LaunchCounts {
 struct Shape {
   int warps = 4;     // per CTA (one item per CTA)
   int ctas = 0;      // resident CTAs per SM
-  int S = 0;         // plates per item in shared memory
-  size_t smem = 0;   // dynamic shared memory per CTA
+  int S = 0;         // plates per item that are the CTA's own
+  size_t smem = 0;   // dynamic shared memory per CTA (their grids, when asked for)
   int n_slots = 0;   // resident CTAs on the GPU (the persistent grid)
 };
 
@@ -1303,11 +1465,19 @@ struct Shape {
 // Fixed device scratch for brkga_decode_noalloc: every GPU that loads this
 // library reserves it until the process exits.  Host code must not use the
 // symbol as an address; brkga_problem_create looks up its device address.
+// The tables and the pool plates' grids go into the first array, their erosion
+// planes and the CTAs' own plates into the second, which is large enough for as
+// many plates as the first can hold grids of (a plane set has four rows for
+// four or eight grid rows, and the CTAs' own grids are at most what shared
+// memory would hold, 34 MB).
 static __device__ __align__(256) unsigned char g_noalloc_scratch[BRKGA_NOALLOC_SCRATCH_BYTES];
+constexpr size_t kNoallocPlaneBytes = (size_t)2 * BRKGA_NOALLOC_SCRATCH_BYTES;
+static __device__ __align__(256) unsigned char g_noalloc_planes[kNoallocPlaneBytes];
 
 struct BrkgaProblem {
   int device = 0;
-  void* noalloc_scratch = nullptr;  // device address of g_noalloc_scratch on `device`
+  void* noalloc_scratch = nullptr;  // device addresses of g_noalloc_scratch and g_noalloc_planes on `device`
+  void* noalloc_planes = nullptr;
   int K = 0;                        // instances
   std::vector<InstDev> inst;
   std::vector<int> s2;              // bitonic sort width per instance
@@ -1317,8 +1487,8 @@ struct BrkgaProblem {
   int req_warps = 0, req_ctas = 0, req_plates = -1;  // requested launch shape (0 / 0 / -1 = automatic)
   int task_max = kDefaultTaskMax;
   Shape shape[3];      // 4, 2 and 1 warps per item
-  int min_S = 0;       // fewest plates in shared memory of the three shapes (pool sizing)
-  int slot_words = 0, slot_vac_off = 0;
+  int min_S = 0;       // fewest own plates per CTA of the three shapes (pool sizing)
+  int grid_words = 0, coarse_words = 0, vac_off = 0;  // words of a plate's grid, of its planes and vacancies, of the planes
   std::vector<MachDev> mach;
   std::vector<void*> allocations;
   Tables tb{};
@@ -1332,8 +1502,11 @@ struct BrkgaProblem {
   int32_t* d_nrot = nullptr;
   int32_t* d_best = nullptr;
   RotDev* d_rot = nullptr;
-  uint32_t* d_vtest = nullptr;
+  CoarseIdx* d_cidx = nullptr;
+  uint2* d_centry = nullptr;
+  uint32_t* d_cfilter = nullptr;
   uint2* d_truns = nullptr;
+  uint2* d_tsegs = nullptr;
   uint32_t* d_maskbits = nullptr;
   uint8_t* d_fits = nullptr;
   uint8_t* d_newbin_ok = nullptr;
@@ -1401,6 +1574,17 @@ int scratch_slots(const BrkgaProblem* pb, int64_t items) {
   return n;
 }
 
+// Plates of their own of a launch's CTAs: the most of any shape that a launch
+// of at most `items` items can use.
+int64_t own_plates(const BrkgaProblem* pb, int64_t items) {
+  auto of = [&](const Shape& s) { return std::min<int64_t>(items, s.n_slots) * s.S; };
+  if (pb->req_warps) return of(pick_shape(pb, items));
+  int64_t n = of(pb->shape[0]);
+  if (items > 3 * (int64_t)pb->shape[0].n_slots) n = std::max(n, of(pb->shape[1]));
+  if (items > 16 * (int64_t)pb->shape[1].n_slots) n = std::max(n, of(pb->shape[2]));
+  return n;
+}
+
 Layout layout_of(const BrkgaProblem* pb, const LaunchCounts& lc, int64_t pool_bins) {
   Layout l;
   size_t o = 0;
@@ -1421,7 +1605,10 @@ Layout layout_of(const BrkgaProblem* pb, const LaunchCounts& lc, int64_t pool_bi
   l.off_bins = o = align_up(o, 256);
   o += (size_t)scratch_slots(pb, lc.items) * std::max(pb->Nmax, 1) * sizeof(BinScal);
   l.off_pool = o = align_up(o, 256);
-  o += (size_t)pool_bins * pb->slot_words * sizeof(uint32_t);
+  o += (size_t)pool_bins * pb->grid_words * sizeof(uint32_t);
+  l.end_pool = l.off_cpool = o = align_up(o, 256);
+  o += (size_t)pool_bins * pb->coarse_words * sizeof(uint32_t);
+  o += (size_t)own_plates(pb, lc.items) * (pb->grid_words + pb->coarse_words) * sizeof(uint32_t);
   l.total = align_up(o, 256);
   return l;
 }
@@ -1482,16 +1669,22 @@ int configure(BrkgaProblem* pb, int warps_req, int ctas_req, int plates_req) {
   cudaDeviceProp prop;
   if (cudaGetDeviceProperties(&prop, pb->device) != cudaSuccess) return BRKGA_ERR_CUDA;
   pb->sm_count = prop.multiProcessorCount;
-  // A plate of machine m uses its own L x RS words, then L vacancy entries:
-  // a slot holds the largest plate of any machine (not Lmax x RSmax, which
-  // for a tall plate beside a wide one is far more than either needs).
-  int Lmax = 0, slot_vac_off = 0;
+  // A plate of machine m uses its own L x RS words, n_planes x NB x RS plane
+  // words and NB vacancies: a slot holds the largest of each of any machine
+  // (not Lmax x RSmax, which for a tall plate beside a wide one is far more
+  // than either needs).
+  int NBmax = 0, Lmax = 0, grid = 0, planes = 0;
   for (const MachDev& m : pb->mach) {
+    NBmax = std::max(NBmax, m.NB);
     Lmax = std::max(Lmax, m.L);
-    slot_vac_off = std::max(slot_vac_off, m.L * m.RS);
+    grid = std::max(grid, m.L * m.RS);
+    planes = std::max(planes, pb->tb.n_planes * m.PS);
   }
-  const int slot_words = (int)align_up((size_t)slot_vac_off + (size_t)(Lmax + 1) / 2, 4);
-  const size_t slot_bytes = (size_t)slot_words * 4;
+  const int grid_words = (int)align_up((size_t)grid, 4);
+  const int coarse_words = (int)align_up((size_t)planes + (size_t)(NBmax + 1) / 2, 4);
+  const size_t grid_bytes = (size_t)grid_words * 4;
+  // room of a plate in shared memory: its grid and two bytes a row
+  const size_t slot_bytes = align_up((size_t)grid + (size_t)(Lmax + 1) / 2, 4) * 4;
   cudaFuncAttributes fa4, fa2, fa1;
   if (cudaFuncGetAttributes(&fa4, decode_kernel<128>) != cudaSuccess ||
       cudaFuncGetAttributes(&fa2, decode_kernel<64>) != cudaSuccess ||
@@ -1534,9 +1727,13 @@ int configure(BrkgaProblem* pb, int warps_req, int ctas_req, int plates_req) {
         while (ctas > 1 && fit_for(ctas) < S) --ctas;
         if (fit_for(ctas) < S) return BRKGA_ERR_INVALID_ARGUMENT;
       } else {
-        // Resident warps matter far more than where the plates live (the
-        // pool stays in L2): as many plates per item in shared memory as
-        // their share holds, none for large plates.
+        // Resident warps matter far more than where the plates live: in L1,
+        // which all of the SM's shared memory then is, the searches' tables
+        // have room beside them (measured with one to four grids, planes or
+        // both per item in shared memory: P200M6, 100 rows, 0.83-0.90 ms
+        // against 0.78, P50M2 0.39-0.42 against 0.39, P100M4 1.09-1.15
+        // against 1.10).  Each CTA has as many plates of its own as grids
+        // would fit in its share, the others come from the pool.
         S = std::min(fit_for(ctas), 4);
       }
     } else {
@@ -1544,7 +1741,7 @@ int configure(BrkgaProblem* pb, int warps_req, int ctas_req, int plates_req) {
       S = preq >= 0 ? preq : std::min(fit_for(ctas), 4);
     }
     if (S > max_fit) return BRKGA_ERR_INVALID_ARGUMENT;
-    const size_t smem = (size_t)S * slot_bytes;
+    const size_t smem = preq > 0 ? (size_t)S * grid_bytes : 0;
     int occ = 0;
     if ((st = occupancy(warps, smem, &occ))) return st;
     if (occ < 1 || (creq > 0 && occ < creq)) return BRKGA_ERR_INVALID_ARGUMENT;
@@ -1554,8 +1751,9 @@ int configure(BrkgaProblem* pb, int warps_req, int ctas_req, int plates_req) {
     shapes[v].ctas = std::max(1, std::min(occ, ctas));
     shapes[v].n_slots = pb->sm_count * shapes[v].ctas;
   }
-  pb->slot_vac_off = slot_vac_off;
-  pb->slot_words = slot_words;
+  pb->grid_words = grid_words;
+  pb->coarse_words = coarse_words;
+  pb->vac_off = planes;
   pb->min_S = shapes[0].S;
   for (int v = 0; v < 3; ++v) {
     pb->shape[v] = shapes[v];
@@ -1615,7 +1813,11 @@ struct Merged {
   std::vector<int32_t> gene_type, nrot, best;
   std::vector<double> thr, pt, pth, area, bin_area;
   std::vector<RotDev> rot;
-  std::vector<uint32_t> vtest;
+  std::vector<CoarseIdx> cidx;
+  std::vector<uint2> centry;
+  std::vector<uint32_t> cfilter;
+  std::vector<uint2> tsegs;
+  int bsh = 0, n_planes = 0;  // rows of a block (2^bsh), erosion planes that some core reads
   std::vector<uint2> truns;
   std::vector<uint32_t> maskbits;
   std::vector<uint8_t> fits, newbin_ok;
@@ -1623,7 +1825,96 @@ struct Merged {
   std::vector<MachDev> mach;
 };
 
-// Append one instance: derived part tables (densities, runs of ones,
+// Rows of the coarse test's blocks (2^shift).  Blocks of eight rows make the
+// planes small and a core count for eight rows; blocks of four leave fewer rows
+// of a small mask outside whole blocks, whose pairs all go to the exact test.
+// Measured (eight / four rows): 14-25 cell masks 0.73 / 0.64 ms, 10-80 cell
+// masks on plates filled more than once 24.5 / 21.5 ms (64 uneven instances)
+// and 4.4 / 4.0 ms (231 parts on three 444 x 244 plates), on plates a quarter
+// full 2.6 / 2.8 ms (P200M6); 10-120 cell masks 5.8 / 6.5 ms (P100M4), 20-240
+// cell masks 20 / 26 ms (P400M8, 1,024 rows).  So four rows for small masks
+// and, up to medium ones, where the parts fill most of the plates.
+int block_shift(const BrkgaProblemDesc* descs, int K) {
+  double parts = 0.0, height = 0.0, fill = 0.0;  // over the genes: mean mask height, mean fill of their instance's plates
+  for (int k = 0; k < K; ++k) {
+    const BrkgaProblemDesc& d = descs[k];
+    double area = 0.0, plates = 0.0;
+    for (int j = 0; j < d.n_genes; ++j) {
+      const int t = d.gene_type[j], nrot = d.part_nrot[t];
+      area += d.part_area[t];
+      for (int r = 0; r < nrot; ++r) height += (double)d.rot_h[t * 4 + r] / nrot;
+    }
+    for (int m = 0; m < d.n_machines; ++m) plates += d.bin_area[m];
+    parts += d.n_genes;
+    fill += plates > 0.0 ? d.n_genes * area / plates : 0.0;
+  }
+  return height < 28.0 * parts || (height < 50.0 * parts && fill >= 0.6 * parts) ? 2 : 3;
+}
+
+// The coarse test's entries of one rotation (see coarse_ok()): for every
+// offset of its top row in a block of plate rows, the blocks it covers
+// whole and the core of each, widest first, then coarse to fine from the
+// bottom (as the rows of the exact test).  Cores shorter than the first plane's
+// runs are left to the exact test.
+void coarse_tables(const std::vector<std::pair<int, int>>& longest, const RotDev& rd, Merged& g) {
+  struct Core {
+    int block, lo, len;
+  };
+  const int rows = 1 << g.bsh;
+  for (int off = 0; off < rows; ++off) {
+    std::vector<Core> cores;
+    for (int i = (rows - off) % rows; i + rows <= rd.h; i += rows) {
+      int lo = 0, hi = rd.w;
+      for (int k = 0; k < rows; ++k) {
+        lo = std::max(lo, longest[i + k].first);
+        hi = std::min(hi, longest[i + k].second);
+      }
+      if (hi - lo >= (1 << kPlaneMin)) cores.push_back({(i + off) >> g.bsh, lo, hi - lo});
+    }
+    std::vector<int> order;
+    const int n = (int)cores.size();
+    if (n) {
+      std::vector<char> used(n, 0);
+      int widest = 0;
+      for (int c = 1; c < n; ++c)
+        if (cores[c].len > cores[widest].len) widest = c;
+      order.push_back(widest);
+      used[widest] = 1;
+      for (int st = 4; st >= 1; st >>= 1)
+        for (int c = n - 1; c >= 0; c -= st)
+          if (!used[c]) {
+            order.push_back(c);
+            used[c] = 1;
+          }
+    }
+    CoarseIdx ci;
+    ci.e = (int)g.centry.size();
+    ci.f = (int)g.cfilter.size();
+    for (int c : order) {
+      const Core& k = cores[c];
+      g.cfilter.push_back(((uint32_t)k.block << 16) | (uint32_t)k.len);
+      for (int at = 0; at < k.len;) {  // pieces of at most two windows of the longest plane
+        int len = std::min(k.len - at, 2 << kPlaneMax), p = kPlaneMin;
+        if (len < (1 << kPlaneMin)) {  // a short last piece: the first plane's window up to the core's end
+          at = k.len - (1 << kPlaneMin);
+          len = 1 << kPlaneMin;
+        }
+        while (p < kPlaneMax && (2 << p) <= len) ++p;
+        g.centry.push_back(make_uint2((uint32_t)(k.lo + at) | ((uint32_t)(len - (1 << p)) << 16),
+                                      (uint32_t)k.block | ((uint32_t)(p - kPlaneMin) << 16)));
+        g.n_planes = std::max(g.n_planes, p - kPlaneMin + 1);
+        at += len;
+      }
+    }
+    if ((g.centry.size() - ci.e) & 1) g.centry.push_back(g.centry.back());
+    ci.ne = (int)g.centry.size() - ci.e;
+    while ((g.cfilter.size() - ci.f) % kVacIlp) g.cfilter.push_back(0u);
+    ci.nf = (int)g.cfilter.size() - ci.f;
+    g.cidx.push_back(ci);
+  }
+}
+
+// Append one instance: derived part tables (runs of ones, block cores,
 // bit-packed rows) with absolute indices, machines, times, flags.
 void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
   const int N = d->n_genes, M = d->n_machines, T = d->n_types;
@@ -1647,10 +1938,9 @@ void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
         rd.w = w;
         rd.mw = (w + 31) / 32;
         rd.mask_base = (int)g.maskbits.size();
-        rd.imax = 0;
-        rd.dmax = 0;
+        int imax = 0, dmax = 0;  // row with the longest run of ones and that length
         std::vector<std::vector<uint32_t>> row_runs(h);
-        std::vector<int> dens(h, 0);
+        std::vector<std::pair<int, int>> longest(h, {0, 0});  // per row: [first, last + 1) of its longest run
         for (int i = 0; i < h; ++i) {
           int best = 0, j = 0;
           while (j < w) {
@@ -1658,15 +1948,17 @@ void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
               const int s = j;
               while (j < w && mk[(size_t)i * w + j]) ++j;
               row_runs[i].push_back((uint32_t)s | ((uint32_t)(j - s) << 16));
-              best = std::max(best, j - s);
+              if (j - s > best) {
+                best = j - s;
+                longest[i] = {s, j};
+              }
             } else {
               ++j;
             }
           }
-          dens[i] = best;
-          if (best > rd.dmax) {
-            rd.dmax = best;
-            rd.imax = i;
+          if (best > dmax) {
+            dmax = best;
+            imax = i;
           }
           for (int wd = 0; wd < rd.mw; ++wd) {
             uint32_t v = 0;
@@ -1681,11 +1973,12 @@ void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
         // soonest; spreading the first tests over the part's height catches
         // a collision higher up without walking every row below it.
         rd.trun = (int)g.truns.size();
+        rd.tseg = (int)g.tsegs.size();
         {
           std::vector<int> order;
           std::vector<char> used(h, 0);
-          order.push_back(rd.imax);
-          used[rd.imax] = 1;
+          order.push_back(imax);
+          used[imax] = 1;
           for (int st = 16; st >= 1; st >>= 1)
             for (int i = h - 1; i >= 0; i -= st)
               if (!used[i]) {
@@ -1693,11 +1986,18 @@ void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
                 used[i] = 1;
               }
           for (int i : order)
-            for (uint32_t r : row_runs[i]) g.truns.push_back(make_uint2(r, (unsigned)i));
-          rd.vt = (int)g.vtest.size();
-          for (int i : order) g.vtest.push_back(((uint32_t)i << 16) | (uint32_t)dens[i]);
+            for (uint32_t r : row_runs[i]) {
+              g.truns.push_back(make_uint2(r, (unsigned)i));
+              const uint32_t s = r & 0xFFFFu, d = r >> 16;
+              for (uint32_t at = 0; at < d; at += 32)
+                g.tsegs.push_back(make_uint2((s + at) | (std::min(32u, d - at) << 16), (unsigned)i));
+            }
         }
         rd.ntrun = (int)g.truns.size() - rd.trun;
+        rd.ntseg = (int)g.tsegs.size() - rd.tseg;
+        coarse_tables(longest, rd, g);
+      } else {
+        g.cidx.resize(g.cidx.size() + ((size_t)1 << g.bsh), CoarseIdx{0, 0, 0, 0});
       }
       g.rot.push_back(rd);
     }
@@ -1712,6 +2012,8 @@ void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
     md.W = d->bin_width[m];
     md.NW = (md.W + 31) / 32;
     md.RS = md.NW + 2;
+    md.NB = (md.L + (1 << g.bsh) - 1) >> g.bsh;
+    md.PS = md.NB * md.RS;
     md.area = d->bin_area[m];
     md.setup = d->setup_time[m];
     g.mach.push_back(md);
@@ -1758,9 +2060,10 @@ void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
 
 // chrom_offs / out_offs (host [K], may be NULL): where each instance's
 // chromosomes (in floats) and makespans start; NULL = packed one after another.
+// cpool: the pool plates' planes, NULL = in the workspace.
 int fill_run(const BrkgaProblem* pb, const int32_t* pops, const int64_t* chrom_offs, const int64_t* out_offs,
              const LaunchCounts& lc, const Layout& l, char* ws, const float* d_chrom, double* d_out,
-             BrkgaPlacement* d_log, int32_t* d_status, int64_t pool_bins, Run* run) {
+             BrkgaPlacement* d_log, int32_t* d_status, int64_t pool_bins, char* cpool, Run* run) {
   std::memset(run, 0, sizeof(Run));
   run->K = pb->K;
   run->n_rows = (int)lc.rows;
@@ -1783,10 +2086,14 @@ int fill_run(const BrkgaProblem* pb, const int32_t* pops, const int64_t* chrom_o
   run->crit_items = pick_shape(pb, lc.items).warps == 4 ? kCritItems : 0;
   run->binscal = reinterpret_cast<BinScal*>(ws + l.off_bins);
   run->pool = reinterpret_cast<uint32_t*>(ws + l.off_pool);
+  run->cpool = reinterpret_cast<uint32_t*>(cpool ? cpool : ws + l.off_cpool);
   run->pool_bins = pool_bins;
   run->S = pick_shape(pb, lc.items).S;
-  run->slot_words = pb->slot_words;
-  run->slot_vac_off = pb->slot_vac_off;
+  run->smem_grids = pick_shape(pb, lc.items).smem > 0;
+  run->own = run->cpool + (size_t)pool_bins * pb->coarse_words;
+  run->grid_words = pb->grid_words;
+  run->coarse_words = pb->coarse_words;
+  run->vac_off = pb->vac_off;
   run->task_max = pb->task_max;
   int64_t row = 0, item = 0, seq = 0, chrom = 0;
   for (int k = 0; k < pb->K; ++k) {
@@ -1823,6 +2130,29 @@ int launch(const BrkgaProblem* pb, int stage, const Run& run, cudaStream_t s) {
   }
   if (stage == 0 || stage == 3) reduce_kernel<<<(run.n_rows + 255) / 256, 256, 0, s>>>(pb->tb, run);
   return cudaGetLastError() == cudaSuccess ? BRKGA_OK : BRKGA_ERR_CUDA;
+}
+
+// brkga_decode_multi_at with the pool plates' planes at d_planes (NULL: in the workspace).
+int decode_at(int32_t stage, const BrkgaProblem* pb, const float* d_chrom, const int64_t* chrom_offsets,
+              const int32_t* pops, double* d_makespan, const int64_t* makespan_offsets, BrkgaPlacement* d_log,
+              int32_t* d_status, void* d_ws, size_t ws_bytes, int64_t pool_bins, void* d_planes, void* stream) {
+  if (!pb || !pops || pool_bins < 0 || stage < 0 || stage > 3) return BRKGA_ERR_INVALID_ARGUMENT;
+  LaunchCounts lc;
+  int st = counts_of(pb, pops, &lc);
+  if (st) return st;
+  for (int k = 0; k < pb->K; ++k)
+    if ((chrom_offsets && chrom_offsets[k] < 0) || (makespan_offsets && makespan_offsets[k] < 0))
+      return BRKGA_ERR_INVALID_ARGUMENT;
+  if (lc.rows == 0) return BRKGA_OK;
+  if (!d_chrom || !d_makespan || !d_status || !d_ws) return BRKGA_ERR_INVALID_ARGUMENT;
+  if (pool_bins == 0) pool_bins = default_pool_bins(pb, lc.items);
+  const Layout l = layout_of(pb, lc, pool_bins);
+  if (ws_bytes < (d_planes ? l.end_pool : l.total)) return BRKGA_ERR_WORKSPACE;
+  DeviceGuard g(pb->device);
+  Run run;
+  fill_run(pb, pops, chrom_offsets, makespan_offsets, lc, l, static_cast<char*>(d_ws), d_chrom, d_makespan, d_log,
+           d_status, pool_bins, static_cast<char*>(d_planes), &run);
+  return launch(pb, stage, run, static_cast<cudaStream_t>(stream));
 }
 
 }  // namespace
@@ -1901,13 +2231,18 @@ int brkga_problem_create_multi(const BrkgaProblemDesc* descs, int32_t K, BrkgaPr
     return BRKGA_ERR_NO_DEVICE;
   }
   Merged g;
+  g.bsh = block_shift(descs, K);
   for (int k = 0; k < K; ++k) merge_instance(&descs[k], g);
-  if (g.maskbits.size() >= ((size_t)1 << 31) || g.truns.size() >= ((size_t)1 << 31)) return BRKGA_ERR_BAD_INSTANCE;
+  if (g.maskbits.size() >= ((size_t)1 << 31) || g.truns.size() >= ((size_t)1 << 31) ||
+      g.centry.size() >= ((size_t)1 << 31))
+    return BRKGA_ERR_BAD_INSTANCE;
   BrkgaProblem* pb = new BrkgaProblem();
   cudaGetDevice(&pb->device);
   pb->K = K;
   pb->inst = g.inst;
   pb->mach = g.mach;
+  pb->tb.bsh = g.bsh;
+  pb->tb.n_planes = g.n_planes;
   for (const InstDev& id : g.inst) {
     int s2 = 1;
     while (s2 < id.N) s2 <<= 1;
@@ -1926,7 +2261,8 @@ int brkga_problem_create_multi(const BrkgaProblemDesc* descs, int32_t K, BrkgaPr
       (st = upload(pb, &pb->d_pt, g.pt)) || (st = upload(pb, &pb->d_pth, g.pth)) ||
       (st = upload(pb, &pb->d_area, g.area)) || (st = upload(pb, &pb->d_nrot, g.nrot)) ||
       (st = upload(pb, &pb->d_best, g.best)) || (st = upload(pb, &pb->d_rot, g.rot)) ||
-      (st = upload(pb, &pb->d_vtest, g.vtest)) || (st = upload(pb, &pb->d_truns, g.truns)) ||
+      (st = upload(pb, &pb->d_tsegs, g.tsegs)) || (st = upload(pb, &pb->d_cidx, g.cidx)) ||
+      (st = upload(pb, &pb->d_centry, g.centry)) || (st = upload(pb, &pb->d_cfilter, g.cfilter)) || (st = upload(pb, &pb->d_truns, g.truns)) ||
       (st = upload(pb, &pb->d_maskbits, g.maskbits)) ||
       (st = upload(pb, &pb->d_fits, g.fits)) || (st = upload(pb, &pb->d_newbin_ok, g.newbin_ok)) ||
       (st = upload(pb, &pb->d_rl, g.rl)) ||
@@ -1945,13 +2281,17 @@ int brkga_problem_create_multi(const BrkgaProblemDesc* descs, int32_t K, BrkgaPr
   tb.nrot = pb->d_nrot;
   tb.best_rot = pb->d_best;
   tb.rot = pb->d_rot;
-  tb.vtest = pb->d_vtest;
+  tb.cidx = pb->d_cidx;
+  tb.centry = pb->d_centry;
+  tb.cfilter = pb->d_cfilter;
   tb.truns = pb->d_truns;
+  tb.tsegs = pb->d_tsegs;
   tb.maskbits = pb->d_maskbits;
   tb.newbin_ok = pb->d_newbin_ok;
   tb.fits = pb->d_fits;
   tb.rl = pb->d_rl;
-  if (cudaGetSymbolAddress(&pb->noalloc_scratch, g_noalloc_scratch) != cudaSuccess) {
+  if (cudaGetSymbolAddress(&pb->noalloc_scratch, g_noalloc_scratch) != cudaSuccess ||
+      cudaGetSymbolAddress(&pb->noalloc_planes, g_noalloc_planes) != cudaSuccess) {
     brkga_problem_destroy(pb);
     return BRKGA_ERR_CUDA;
   }
@@ -1996,7 +2336,7 @@ int brkga_get_launch_config(const BrkgaProblem* pb, int64_t items, int32_t* warp
   const Shape& sh = pick_shape(pb, items);
   if (warps_per_item) *warps_per_item = sh.warps;
   if (ctas_per_sm) *ctas_per_sm = sh.ctas;
-  if (smem_plates) *smem_plates = sh.S;
+  if (smem_plates) *smem_plates = sh.smem ? sh.S : 0;
   if (resident_ctas) *resident_ctas = sh.n_slots;
   if (task_max) *task_max = pb->task_max;
   return BRKGA_OK;
@@ -2021,23 +2361,8 @@ int brkga_decode_multi_at(int32_t stage, const BrkgaProblem* pb, const float* d_
                           const int32_t* pops, double* d_makespan, const int64_t* makespan_offsets,
                           BrkgaPlacement* d_log, int32_t* d_status, void* d_ws, size_t ws_bytes, int64_t pool_bins,
                           void* stream) {
-  if (!pb || !pops || pool_bins < 0 || stage < 0 || stage > 3) return BRKGA_ERR_INVALID_ARGUMENT;
-  LaunchCounts lc;
-  int st = counts_of(pb, pops, &lc);
-  if (st) return st;
-  for (int k = 0; k < pb->K; ++k)
-    if ((chrom_offsets && chrom_offsets[k] < 0) || (makespan_offsets && makespan_offsets[k] < 0))
-      return BRKGA_ERR_INVALID_ARGUMENT;
-  if (lc.rows == 0) return BRKGA_OK;
-  if (!d_chrom || !d_makespan || !d_status || !d_ws) return BRKGA_ERR_INVALID_ARGUMENT;
-  if (pool_bins == 0) pool_bins = default_pool_bins(pb, lc.items);
-  const Layout l = layout_of(pb, lc, pool_bins);
-  if (ws_bytes < l.total) return BRKGA_ERR_WORKSPACE;
-  DeviceGuard g(pb->device);
-  Run run;
-  fill_run(pb, pops, chrom_offsets, makespan_offsets, lc, l, static_cast<char*>(d_ws), d_chrom, d_makespan, d_log,
-           d_status, pool_bins, &run);
-  return launch(pb, stage, run, static_cast<cudaStream_t>(stream));
+  return decode_at(stage, pb, d_chrom, chrom_offsets, pops, d_makespan, makespan_offsets, d_log, d_status, d_ws,
+                   ws_bytes, pool_bins, nullptr, stream);
 }
 
 int brkga_decode_multi_stage(int32_t stage, const BrkgaProblem* pb, const float* d_chrom, const int32_t* pops,
@@ -2081,11 +2406,14 @@ int brkga_decode_noalloc(const BrkgaProblem* pb, const float* d_chrom, int32_t P
   if (counts_of(pb, &P, &lc)) return BRKGA_ERR_INVALID_ARGUMENT;
   const Layout fixed = layout_of(pb, lc, 0);  // offsets up to the pool do not depend on the pool size
   if (fixed.off_pool >= cap) return BRKGA_ERR_WORKSPACE;
-  int64_t pool_bins = (int64_t)((cap - fixed.off_pool) / ((size_t)pb->slot_words * sizeof(uint32_t)));
-  while (pool_bins > 0 && layout_of(pb, lc, pool_bins).total > cap) --pool_bins;  // 256-byte rounding
+  const size_t own = (size_t)own_plates(pb, lc.items) * (pb->grid_words + pb->coarse_words) * 4;
+  if (own >= kNoallocPlaneBytes) return BRKGA_ERR_WORKSPACE;
+  const int64_t planes = (int64_t)((kNoallocPlaneBytes - own) / ((size_t)pb->coarse_words * 4));
+  int64_t pool_bins = std::min((int64_t)((cap - fixed.off_pool) / ((size_t)pb->grid_words * 4)), planes);
+  while (pool_bins > 0 && layout_of(pb, lc, pool_bins).end_pool > cap) --pool_bins;  // 256-byte rounding
   if (pool_bins < 1) return BRKGA_ERR_WORKSPACE;
-  return brkga_decode_stage(0, pb, d_chrom, P, d_makespan, d_log, d_status, pb->noalloc_scratch, cap,
-                            pool_bins, stream);
+  return decode_at(0, pb, d_chrom, nullptr, &P, d_makespan, nullptr, d_log, d_status, pb->noalloc_scratch, cap,
+                   pool_bins, pb->noalloc_planes, stream);
 }
 
 int brkga_evaluate_host(BrkgaProblem* pb, const float* h_chrom, int32_t P, double* h_makespan,
@@ -2194,7 +2522,9 @@ int brkga_initial_solution_host(BrkgaProblem* pb, const int32_t* h_order, int32_
   const size_t off_ctr = o;
   o = align_up(o + 64, 256);
   const size_t off_pool = o;
-  o = align_up(o + (size_t)nn * pb->slot_words * 4, 256);
+  o = align_up(o + (size_t)nn * pb->grid_words * 4, 256);
+  const size_t off_cpool = o;
+  o = align_up(o + (size_t)nn * pb->coarse_words * 4, 256);
   const size_t state_bytes = align_up(greedy_state_bytes(nn, pb->M), 256);
   const bool in_smem = state_bytes <= kGreedyMaxSmem - 4096;
   const size_t off_state = o;
@@ -2222,8 +2552,10 @@ int brkga_initial_solution_host(BrkgaProblem* pb, const int32_t* h_order, int32_
     g.status = reinterpret_cast<int32_t*>(d + off_ctr + 40);
     g.binscal = reinterpret_cast<BinScal*>(d + off_bs);
     g.pool = reinterpret_cast<uint32_t*>(d + off_pool);
-    g.slot_words = pb->slot_words;
-    g.slot_vac_off = pb->slot_vac_off;
+    g.cpool = reinterpret_cast<uint32_t*>(d + off_cpool);
+    g.grid_words = pb->grid_words;
+    g.coarse_words = pb->coarse_words;
+    g.vac_off = pb->vac_off;
     g.order = reinterpret_cast<const int32_t*>(d + off_order);
     g.n = n;
     g.out_machine = reinterpret_cast<int32_t*>(d + off_mach);
