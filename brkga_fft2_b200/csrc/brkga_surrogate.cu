@@ -96,13 +96,24 @@ struct FeatParams {
   const double* thr;
   const int32_t* gene_type;
   const double* part_area;
-  const double* pt;
   const double* pth;
-  const double* bin_area;
-  float inv_pt, inv_pth;  // 1 / max proc time, 1 / max height time
+  const float4* shares;   // [machine * T + type], see ShareTable
+  float inv_pth;          // 1 / max height time
   __nv_bfloat16* X;       // [rows, in_pad]
   int row_offset;
 };
+
+// What a part adds to a feature row on a machine, made once per surrogate:
+// x = its share of the plate's area, y = its processing time and z = its height
+// time, each over the instance's largest.  (Per row and part these cost a
+// float64 division and two conversions.)
+__global__ void share_table_kernel(const double* part_area, const double* bin_area, const double* pt, const double* pth,
+                                   int M, int T, float inv_pt, float inv_pth, float4* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= M * T) return;
+  const int m = i / T, t = i - m * T;
+  out[i] = make_float4((float)(part_area[t] / bin_area[m]), (float)pt[i] * inv_pt, (float)pth[i] * inv_pth, 0.f);
+}
 
 // One CTA per chromosome: sort (machine, key, gene) like the decoder, write the
 // feature row.  Per-machine sums run in decode order, so features are deterministic.
@@ -163,9 +174,9 @@ __global__ void features_kernel(FeatParams p) {
       const int m = (int)(key >> 48);
       float av = 0.f, lv = 0.f;
       if (m < p.M) {
-        const int t = p.gene_type[(int)(key & 0xFFFFu)];
-        av = (float)(p.part_area[t] / p.bin_area[m]);
-        lv = (float)p.pt[(size_t)m * p.T + t] * p.inv_pt;
+        const float4 sv = p.shares[(size_t)m * p.T + p.gene_type[(int)(key & 0xFFFFu)]];
+        av = sv.x;
+        lv = sv.y;
       }
       c_area[q] = av;
       c_load[q] = lv;
@@ -202,10 +213,9 @@ __global__ void features_kernel(FeatParams p) {
       const unsigned long long key = keys[i / 3];
       const int m = (int)(key >> 48);
       if (m < p.M) {
-        const int t = p.gene_type[(int)(key & 0xFFFFu)];
+        const float4 sv = p.shares[(size_t)m * p.T + p.gene_type[(int)(key & 0xFFFFu)]];
         const int f = i % 3;
-        v = f == 0 ? (float)m * mscale
-                   : f == 1 ? (float)p.pt[(size_t)m * p.T + t] * p.inv_pt : (float)p.pth[(size_t)m * p.T + t] * p.inv_pth;
+        v = f == 0 ? (float)m * mscale : f == 1 ? sv.y : sv.z;
       }
     } else if (i < 3 * p.N + 2 * p.M) {
       const int q = i - 3 * p.N;
@@ -219,11 +229,17 @@ __global__ void features_kernel(FeatParams p) {
 // most 32 machines: the warp sorts the (machine, key, gene) keys in
 // registers (E per lane, bitonic network, partners in other lanes exchanged
 // by shuffles; no CTA barrier), then works from its own slice of shared
-// memory.  Same keys, same order of the per-machine sums, same values as
+// memory, where it also puts the row together to store it in 16-byte pieces.
+// Same keys, same order of the per-machine sums, same values as
 // features_kernel: the rows are identical.
+// Six warps per scheduler in one wave, so what bounds it is the instructions a
+// row takes.  With the sort's steps written out (their directions are constants
+// or one lane test), the shares read from their table and whole-row stores
+// 3,600 P100M4 rows take 13.8 us; with the steps in loops, a float64 division
+// per part and a lane per value 22.8 us (a prediction of them 32.6 and 41.6 us).
 constexpr int kFeatWarps = 8;  // warps (chromosomes) per CTA
-__host__ __device__ constexpr size_t feat_warp_bytes(int E) {
-  return (size_t)32 * E * 8 + (size_t)32 * E * 12 + 4 * 33 * 4;  // keys, shares + types, per-machine arrays
+__host__ __device__ constexpr size_t feat_warp_bytes(int E, int in_pad) {
+  return (size_t)32 * E * (8 + 8) + 36 * 4 + (size_t)in_pad * 2;  // keys, shares; first positions; row
 }
 template <int E>
 __global__ void __launch_bounds__(32 * kFeatWarps) features_warp_kernel(FeatParams p) {
@@ -234,14 +250,11 @@ __global__ void __launch_bounds__(32 * kFeatWarps) features_warp_kernel(FeatPara
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c = blockIdx.x * kFeatWarps + warp;
   if (c >= p.P) return;
-  unsigned char* base = fsm + (size_t)warp * feat_warp_bytes(E);
+  unsigned char* base = fsm + (size_t)warp * feat_warp_bytes(E, p.in_pad);
   unsigned long long* keys = reinterpret_cast<unsigned long long*>(base);
-  float* c_area = reinterpret_cast<float*>(keys + S2);
-  float* c_load = c_area + S2;
-  int* c_type = reinterpret_cast<int*>(c_load + S2);
-  int* m_start = c_type + S2;  // [33]
-  float* m_area = reinterpret_cast<float*>(m_start + 33);
-  float* m_load = m_area + 33;
+  float2* c_share = reinterpret_cast<float2*>(keys + S2);  // area, time
+  int* m_start = reinterpret_cast<int*>(c_share + S2);                   // [33], padded to 36
+  __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(m_start + 36);  // [in_pad]
   const float* ch = p.chrom + (size_t)c * 2 * p.N;
   const bool order = p.kind == BRKGA_SURROGATE_FEATURES_ORDER;
   unsigned long long k[E];
@@ -255,33 +268,28 @@ __global__ void __launch_bounds__(32 * kFeatWarps) features_warp_kernel(FeatPara
     }
   }
   // bitonic sort of S2 keys, element i = lane * E + e
-#pragma unroll 1
+#pragma unroll
   for (int kk = 2; kk <= S2; kk <<= 1) {
-#pragma unroll 1
+#pragma unroll
     for (int j = kk >> 1; j > 0; j >>= 1) {
       if (j >= E) {  // partner in lane ^ (j / E), same register
         const int dl = j / E;
+        // kk > j >= E, so the direction is the lane's alone; keep the smaller key where it matches the lane's side
+        const bool keep_min = ((lane & (kk / E)) == 0) == ((lane & dl) == 0);
 #pragma unroll
         for (int e = 0; e < E; ++e) {
-          const int i = lane * E + e;
           const unsigned long long o = __shfl_xor_sync(0xFFFFFFFFu, k[e], dl);
-          const bool asc = (i & kk) == 0, lower = (i & j) == 0;
-          k[e] = (asc == lower) ? (k[e] < o ? k[e] : o) : (k[e] > o ? k[e] : o);
+          k[e] = (k[e] < o) == keep_min ? k[e] : o;
         }
       } else {  // partner in the same lane
 #pragma unroll
         for (int e = 0; e < E; ++e) {
-#pragma unroll
-          for (int jj = 1; jj < E; jj <<= 1) {
-            if (jj == j && (e & jj) == 0) {
-              const int i = lane * E + e;
-              const bool asc = (i & kk) == 0;
-              const unsigned long long a = k[e], b = k[e | jj];
-              if ((a > b) == asc) {
-                k[e] = b;
-                k[e | jj] = a;
-              }
-            }
+          if ((e & j) == 0) {
+            const bool asc = kk < E ? (e & kk) == 0 : (lane & (kk / E)) == 0;
+            const unsigned long long a = k[e], b = k[e | j];
+            const bool swap = (a > b) == asc;
+            k[e] = swap ? b : a;
+            k[e | j] = swap ? a : b;
           }
         }
       }
@@ -300,62 +308,45 @@ __global__ void __launch_bounds__(32 * kFeatWarps) features_warp_kernel(FeatPara
     }
     m_start[m] = lo;
   }
+  const float mscale = p.M > 1 ? 1.f / (float)(p.M - 1) : 0.f;
   for (int q = lane; q < p.N; q += 32) {
     const unsigned long long key = keys[q];
-    const int m = (int)(key >> 48);
-    float av = 0.f, lv = 0.f;
-    int t = -1;
-    if (m < p.M) {
-      t = p.gene_type[(int)(key & 0xFFFFu)];
-      if (!order) {
-        av = (float)(p.part_area[t] / p.bin_area[m]);
-        lv = (float)p.pt[(size_t)m * p.T + t] * p.inv_pt;
-      }
+    const int m = (int)(key >> 48), g = (int)(key & 0xFFFFu);
+    float2 share = make_float2(0.f, 0.f);
+    float v0 = 0.f, v1 = 0.f, v2 = 0.f;
+    if (order) {
+      const int t = p.gene_type[g];
+      v0 = ch[g];
+      v1 = (float)p.part_area[t] * p.inv_area;
+      v2 = (float)p.pth[t] * p.inv_pth;
+    } else if (m < p.M) {
+      const float4 sv = p.shares[(size_t)m * p.T + p.gene_type[g]];
+      share = make_float2(sv.x, sv.y);
+      v0 = (float)m * mscale;
+      v1 = sv.y;
+      v2 = sv.z;
     }
-    c_area[q] = av;
-    c_load[q] = lv;
-    c_type[q] = t;
+    c_share[q] = share;
+    out[3 * q] = __float2bfloat16(v0);
+    out[3 * q + 1] = __float2bfloat16(v1);
+    out[3 * q + 2] = __float2bfloat16(v2);
   }
   __syncwarp();
+  const int used = order ? 3 * p.N : 3 * p.N + 2 * p.M;
   if (!order && lane < p.M) {  // per machine, in decode order
     float area = 0.f, load = 0.f;
     for (int q = m_start[lane]; q < m_start[lane + 1]; ++q) {
-      area += c_area[q];
-      load += c_load[q];
+      const float2 share = c_share[q];
+      area += share.x;
+      load += share.y;
     }
-    m_area[lane] = area;
-    m_load[lane] = load;
+    out[3 * p.N + 2 * lane] = __float2bfloat16(area);
+    out[3 * p.N + 2 * lane + 1] = __float2bfloat16(load);
   }
+  for (int i = used + lane; i < p.in_pad; i += 32) out[i] = __float2bfloat16(0.f);
   __syncwarp();
-  __nv_bfloat16* row = p.X + (size_t)(p.row_offset + c) * p.in_pad;
-  if (order) {
-    for (int i = lane; i < p.in_pad; i += 32) {
-      float v = 0.f;
-      if (i < 3 * p.N) {
-        const int q = i / 3, f = i - 3 * q, g = (int)(keys[q] & 0xFFFFu), t = c_type[q];
-        v = f == 0 ? ch[g] : f == 1 ? (float)p.part_area[t] * p.inv_area : (float)p.pth[t] * p.inv_pth;
-      }
-      row[i] = __float2bfloat16(v);
-    }
-    return;
-  }
-  const float mscale = p.M > 1 ? 1.f / (float)(p.M - 1) : 0.f;
-  for (int i = lane; i < p.in_pad; i += 32) {
-    float v = 0.f;
-    if (i < 3 * p.N) {
-      const int q = i / 3, f = i - 3 * q;
-      const int m = (int)(keys[q] >> 48);
-      if (m < p.M) {
-        const int t = c_type[q];
-        v = f == 0 ? (float)m * mscale
-                   : f == 1 ? (float)p.pt[(size_t)m * p.T + t] * p.inv_pt : (float)p.pth[(size_t)m * p.T + t] * p.inv_pth;
-      }
-    } else if (i < 3 * p.N + 2 * p.M) {
-      const int q = i - 3 * p.N;
-      v = (q & 1) ? m_load[q >> 1] : m_area[q >> 1];
-    }
-    row[i] = __float2bfloat16(v);
-  }
+  uint4* row = reinterpret_cast<uint4*>(p.X + (size_t)(p.row_offset + c) * p.in_pad);  // in_pad is a multiple of 64
+  for (int i = lane; i < p.in_pad / 8; i += 32) row[i] = reinterpret_cast<const uint4*>(out)[i];
 }
 
 // Launch with programmatic stream serialisation: the kernel may begin while
@@ -754,12 +745,12 @@ struct BrkgaSurrogate {
   int in = 0, in_pad = 0, max_batch = 0, cap = 0;
   uint64_t seed = 0;
   float inv_pt = 1.f, inv_pth = 1.f;
+  float4* shares = nullptr;  // [machine * T + type], share_table_kernel
   const double* thr = nullptr;
   const int32_t* gene_type = nullptr;
   const double* part_area = nullptr;
   const double* pt = nullptr;
   const double* pth = nullptr;
-  const double* bin_area = nullptr;
   std::vector<void*> allocs;
   // parameters (fp32 master), gradients, Adam moments: one flat block each
   float *W1, *b1, *W2, *b2, *w3, *b3;
@@ -893,10 +884,8 @@ int features(BrkgaSurrogate* s, const float* d_chrom, int P, __nv_bfloat16* X, c
   fp.thr = s->thr;
   fp.gene_type = s->gene_type;
   fp.part_area = s->part_area;
-  fp.pt = s->pt;
   fp.pth = s->pth;
-  fp.bin_area = s->bin_area;
-  fp.inv_pt = s->inv_pt;
+  fp.shares = s->shares;
   fp.inv_pth = s->inv_pth;
   fp.kind = s->features_kind;
   fp.inv_area = s->inv_area;
@@ -906,10 +895,10 @@ int features(BrkgaSurrogate* s, const float* d_chrom, int P, __nv_bfloat16* X, c
   while (S2 < s->N) S2 <<= 1;
   if (s->M <= 32 && S2 <= 256) {  // one warp per chromosome
     const dim3 grid((P + kFeatWarps - 1) / kFeatWarps), block(32 * kFeatWarps);
-    if (S2 <= 32) launch_pdl(features_warp_kernel<1>, grid, block, kFeatWarps * feat_warp_bytes(1), st, fp);
-    else if (S2 <= 64) launch_pdl(features_warp_kernel<2>, grid, block, kFeatWarps * feat_warp_bytes(2), st, fp);
-    else if (S2 <= 128) launch_pdl(features_warp_kernel<4>, grid, block, kFeatWarps * feat_warp_bytes(4), st, fp);
-    else launch_pdl(features_warp_kernel<8>, grid, block, kFeatWarps * feat_warp_bytes(8), st, fp);
+    if (S2 <= 32) launch_pdl(features_warp_kernel<1>, grid, block, kFeatWarps * feat_warp_bytes(1, s->in_pad), st, fp);
+    else if (S2 <= 64) launch_pdl(features_warp_kernel<2>, grid, block, kFeatWarps * feat_warp_bytes(2, s->in_pad), st, fp);
+    else if (S2 <= 128) launch_pdl(features_warp_kernel<4>, grid, block, kFeatWarps * feat_warp_bytes(4, s->in_pad), st, fp);
+    else launch_pdl(features_warp_kernel<8>, grid, block, kFeatWarps * feat_warp_bytes(8, s->in_pad), st, fp);
   } else {
     launch_pdl(features_kernel, P, std::min(1024, std::max(64, S2 / 2)), features_smem(S2, s->N), st, fp);
   }
@@ -1077,7 +1066,6 @@ int brkga_surrogate_create_ex(const BrkgaProblem* problem, int32_t max_batch, in
     delete s;
     return BRKGA_ERR_INVALID_ARGUMENT;
   }
-  s->bin_area = bin_area;
   s->in = features == BRKGA_SURROGATE_FEATURES_ORDER ? 3 * s->N : 3 * s->N + 2 * s->M;
   s->in_pad = round_up(s->in, 64);
   s->max_batch = max_batch;
@@ -1103,7 +1091,7 @@ int brkga_surrogate_create_ex(const BrkgaProblem* problem, int32_t max_batch, in
     s->inv_area = ma > 0 ? (float)(1.0 / ma) : 1.f;
   }
   if (cudaFuncSetAttribute(features_warp_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)(kFeatWarps * feat_warp_bytes(8))) != cudaSuccess ||
+                           (int)(kFeatWarps * feat_warp_bytes(8, round_up(3 * 256 + 2 * 32, 64)))) != cudaSuccess ||
       cudaFuncSetAttribute(features_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)features_smem(kMaxGenes, kMaxGenes)) !=
           cudaSuccess ||
@@ -1127,10 +1115,13 @@ int brkga_surrogate_create_ex(const BrkgaProblem* problem, int32_t max_batch, in
       (st = dalloc(s, &s->outp, (size_t)(kMaxTrainBatch / 32) * (2 * kH2 + 2))) || (st = dalloc(s, &s->dH1, (size_t)B * kH1)) || (st = dalloc(s, &s->loss, 1)) ||
       (st = dalloc(s, &s->n_valid, 1)) || (st = dalloc(s, &s->slot, B)) || (st = dalloc(s, &s->err, 1)) || (st = dalloc(s, &s->count, 1)) ||
       (st = dalloc(s, &s->step, 1)) || (st = dalloc(s, &s->adam_t, 1)) || (st = dalloc(s, &s->norm, 3)) ||
-      (st = dalloc(s, &s->bufX, (size_t)s->cap * I)) || (st = dalloc(s, &s->bufY, s->cap))) {
+      (st = dalloc(s, &s->bufX, (size_t)s->cap * I)) || (st = dalloc(s, &s->bufY, s->cap)) ||
+      (st = dalloc(s, &s->shares, (size_t)s->M * s->T))) {
     brkga_surrogate_destroy(s);
     return st;
   }
+  share_table_kernel<<<(s->M * s->T + 255) / 256, 256>>>(s->part_area, bin_area, s->pt, s->pth, s->M, s->T, s->inv_pt,
+                                                         s->inv_pth, s->shares);
   float* q = s->params;
   s->W1 = q; q += nW1; s->b1 = q; q += kH1; s->W2 = q; q += nW2; s->b2 = q; q += kH2; s->w3 = q; q += kH2; s->b3 = q;
   q = s->grads;
