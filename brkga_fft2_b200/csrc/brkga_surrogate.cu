@@ -45,6 +45,7 @@ namespace {
 constexpr int kH1 = 512;
 constexpr int kH2 = 256;
 constexpr int kMaxGenes = 8192;
+constexpr int kSms = 148;
 constexpr int kMaxTrainBatch = 16384;  // rows of one gradient step (sizes the backward pass's row-block partials)
 
 struct U4 {
@@ -798,7 +799,9 @@ int prepare_gemm() {
   if (cudaFuncSetAttribute(umma::gemm_bf16_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            umma::gemm_smem_bytes<128>()) != cudaSuccess ||
       cudaFuncSetAttribute(umma::gemm_bf16_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           umma::gemm_smem_bytes<64>()) != cudaSuccess)
+                           umma::gemm_smem_bytes<64>()) != cudaSuccess ||
+      cudaFuncSetAttribute(umma::gemm_bf16_kernel<64, umma::kManyTilesStages>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           umma::gemm_smem_bytes<64, umma::kManyTilesStages>()) != cudaSuccess)
     return BRKGA_ERR_CUDA;
   ready[dev] = 1;
   return BRKGA_OK;
@@ -806,7 +809,7 @@ int prepare_gemm() {
 
 // 128 x 128 tiles when they alone fill the GPU twice over, else 128 x 64
 // (these GEMMs are small: more CTAs matter more than tile reuse).
-int tile_n(int M, int N) { return (N % 128 == 0 && (long long)(M / 128) * (N / 128) >= 2 * 148) ? 128 : 64; }
+int tile_n(int M, int N) { return (N % 128 == 0 && (long long)(M / 128) * (N / 128) >= 2 * kSms) ? 128 : 64; }
 
 // cuTensorMapEncodeTiled from the driver, looked up once per process through
 // the runtime (no link against libcuda).
@@ -853,6 +856,9 @@ int gemm(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, const
   if (bn == 128) {
     launch_pdl(umma::gemm_bf16_kernel<128>, dim3(M / 128, N / 128), 128, umma::gemm_smem_bytes<128>(), st, ta, tb,
                ep, K, err);
+  } else if ((long long)(M / 128) * (N / 64) > kSms) {
+    launch_pdl(umma::gemm_bf16_kernel<64, umma::kManyTilesStages>, dim3(M / 128, N / 64), 128,
+               umma::gemm_smem_bytes<64, umma::kManyTilesStages>(), st, ta, tb, ep, K, err);
   } else {
     launch_pdl(umma::gemm_bf16_kernel<64>, dim3(M / 128, N / 64), 128, umma::gemm_smem_bytes<64>(), st, ta, tb, ep,
                K, err);

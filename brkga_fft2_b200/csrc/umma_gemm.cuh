@@ -70,18 +70,22 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
 }
 
 // Stages of A and B tiles in shared memory (24 KB per stage at BN = 64,
-// 32 KB at BN = 128): enough that the copies of every K step of the
-// surrogate's GEMMs (K <= 640) are in flight at once.
+// 32 KB at BN = 128).  A GEMM of at most one CTA per SM takes as many as fit,
+// so that the copies of most K steps are in flight at once (a training step of
+// 512 rows, K up to 512: 54 us, with four stages 56).  One of more tiles takes
+// four, two CTAs per SM, instead of a second wave: a prediction of 3,600 rows
+// (232 and 116 tiles) 29.2 us against 33.2, of 8,000 rows 41.4 against 53.7.
 template <int BN>
 __host__ __device__ constexpr int gemm_stages() {
   return BN == 128 ? 5 : 6;
 }
+constexpr int kManyTilesStages = 4;
 
-// Dynamic shared memory of gemm_bf16_kernel<BN>: the stages plus 1 KB to
+// Dynamic shared memory of gemm_bf16_kernel<BN, kSt>: the stages plus 1 KB to
 // align them on the swizzle's 1024-byte period.
-template <int BN>
+template <int BN, int kSt = gemm_stages<BN>()>
 __host__ __device__ constexpr int gemm_smem_bytes() {
-  return gemm_stages<BN>() * (kTileM * kTileK + BN * kTileK) * 2 + 1024;
+  return kSt * (kTileM * kTileK + BN * kTileK) * 2 + 1024;
 }
 
 // Programmatic dependent launch: a kernel launched with programmatic stream
@@ -148,12 +152,11 @@ struct Epilogue {
 //              after the last step one more commit signals "acc";
 //   all warps  wait for "acc" and run the epilogue from tensor memory.
 // No multicast; every wait is bounded (the error path is in the kernel).
-template <int BN>
+template <int BN, int kSt = gemm_stages<BN>()>
 __global__ void __launch_bounds__(128) gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA,
                                                         const __grid_constant__ CUtensorMap tmB,
                                                         const __grid_constant__ Epilogue ep, int K, int* err) {
   static_assert(BN == 64 || BN == 128, "BN must be 64 or 128");
-  constexpr int kSt = gemm_stages<BN>();
   constexpr int kCols = BN;  // tensor-memory columns (power of two >= 32)
   constexpr uint32_t kABytes = kTileM * kTileK * 2, kBBytes = BN * kTileK * 2, kStageBytes = kABytes + kBBytes;
   extern __shared__ uint8_t smem_raw[];
