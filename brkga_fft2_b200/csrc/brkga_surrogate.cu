@@ -695,28 +695,53 @@ __global__ void observe_kernel(ObsParams p, const int* slot) {
   if (threadIdx.x == 0) p.bufY[sl] = (float)((p.makespan[r] - p.norm[0]) / p.norm[1]);
 }
 
-// Minibatch: uniform rows of the filled part of the ring buffer.
-__global__ void gather_kernel(const __nv_bfloat16* bufX, const float* bufY, const long long* count, int cap, int B,
-                              int n_valid_max, int in_pad, uint32_t k0, uint32_t k1, const long long* step,
-                              __nv_bfloat16* X, __nv_bfloat16* XT, float* y, int* n_valid) {
+// Minibatch: uniform rows of the filled part of the ring buffer, row-major and
+// transposed.  Tiles of 32 rows x 64 columns through shared memory, so that the
+// loads and both stores are whole pieces of at least 64 bytes: with a CTA per
+// row, whose transposed stores were two bytes each, six training steps of 512
+// rows took 324 us, now 313 (of 1,024 rows 384 and 366).
+__global__ void __launch_bounds__(256) gather_kernel(const __nv_bfloat16* bufX, const float* bufY, const long long* count,
+                                                     int cap, int B, int n_valid_max, int in_pad, uint32_t k0, uint32_t k1,
+                                                     const long long* step, __nv_bfloat16* X, __nv_bfloat16* XT, float* y,
+                                                     int* n_valid) {
   umma::pdl_wait();
   umma::pdl_trigger();
-  const int b = blockIdx.x;
+  __shared__ int s_src[32];
+  __shared__ uint32_t s_t[32][33];  // [column pair][row]
+  const int tid = threadIdx.x, b0 = blockIdx.x * 32, c0 = blockIdx.y * 64;
   const long long filled = min((long long)cap, *count);
   const int nv = (int)min((long long)n_valid_max, filled);
-  if (b == 0 && threadIdx.x == 0) *n_valid = nv;
-  const bool real = b < nv && filled > 0;
-  int src = 0;
-  if (real) {
-    const U4 r = philox(U4{(uint32_t)b, (uint32_t)(*step), 0x6A7u, 0u}, k0, k1);
-    src = (int)mulhi32(r.x, (uint32_t)filled);
+  if (tid < 32) {
+    const int b = b0 + tid;
+    int src = -1;
+    if (b < nv && filled > 0) {
+      const U4 r = philox(U4{(uint32_t)b, (uint32_t)(*step), 0x6A7u, 0u}, k0, k1);
+      src = (int)mulhi32(r.x, (uint32_t)filled);
+    }
+    s_src[tid] = src;
+    if (blockIdx.y == 0) {
+      y[b] = src >= 0 ? bufY[src] : 0.f;
+      if (b == 0) *n_valid = nv;
+    }
   }
-  for (int i = threadIdx.x; i < in_pad; i += blockDim.x) {
-    const __nv_bfloat16 q = real ? bufX[(size_t)src * in_pad + i] : __float2bfloat16(0.f);
-    X[(size_t)b * in_pad + i] = q;
-    XT[(size_t)i * B + b] = q;
+  __syncthreads();
+  const int tx = tid & 31, ty = tid >> 5;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int r = ty + 8 * q, src = s_src[r];
+    const uint32_t v =
+        src >= 0 ? *reinterpret_cast<const uint32_t*>(bufX + (size_t)src * in_pad + c0 + 2 * tx) : 0u;
+    *reinterpret_cast<uint32_t*>(X + (size_t)(b0 + r) * in_pad + c0 + 2 * tx) = v;
+    s_t[tx][r] = v;
   }
-  if (threadIdx.x == 0) y[b] = real ? bufY[src] : 0.f;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {  // column pair ty + 8q, row tx
+    const uint32_t v = s_t[ty + 8 * q][tx];
+    const int c = c0 + 2 * (ty + 8 * q);
+    reinterpret_cast<uint16_t*>(XT)[(size_t)c * B + b0 + tx] = (uint16_t)(v & 0xFFFFu);
+    reinterpret_cast<uint16_t*>(XT)[(size_t)(c + 1) * B + b0 + tx] = (uint16_t)(v >> 16);
+  }
 }
 
 __global__ void bump_kernel(long long* step) { *step += 1; }
@@ -1227,7 +1252,7 @@ int brkga_surrogate_train(BrkgaSurrogate* s, int32_t steps, int32_t batch, float
   // layer's backward pass (which also advances the step counters), three
   // backward GEMMs, one column reduction, Adam with the bf16 casts
   for (int i = 0; i < steps; ++i) {
-    launch_pdl(gather_kernel, batch, 128, 0, st, s->bufX, s->bufY, s->count, s->cap, batch, batch, s->in_pad,
+    launch_pdl(gather_kernel, dim3(batch / 32, s->in_pad / 64), 256, 0, st, s->bufX, s->bufY, s->count, s->cap, batch, batch, s->in_pad,
                (uint32_t)s->seed, (uint32_t)(s->seed >> 32), s->step, s->X, s->XT, s->t, s->n_valid);
     if ((r = gradients(s, batch, 1, st))) return r;
     if ((r = adam_cast(s, lr, true, st))) return r;
