@@ -148,7 +148,8 @@ int brkga_decode_stage(int32_t stage, const BrkgaProblem* problem, const float* 
  * because those can synchronise the device.  No reference counterpart: the
  * reference grows its workspaces as it goes.
  * Same inputs and outputs as brkga_decode, but the workspace is a fixed
- * 64 MiB array inside the library, so nothing is allocated or freed here.
+ * 64 MiB array inside the library (and one of 128 MiB beside it for what the
+ * search derives from the plates), so nothing is allocated or freed here.
  * Its device address is looked up by brkga_problem_create (set-up, with the
  * problem's device current).  The per-population tables must fit in it
  * (else BRKGA_ERR_WORKSPACE, before any launch); the plate pool gets the rest,
@@ -220,16 +221,21 @@ int brkga_decode_multi_at(int32_t stage, const BrkgaProblem* problem, const floa
  *                   per CTA; 0 = automatic per launch (4 while the items fill
  *                   at most three waves of resident 4-warp CTAs, where the
  *                   latency of one item dominates; 2 up to sixteen waves of
- *                   2-warp CTAs; 1 beyond, where throughput does)
+ *                   2-warp CTAs; 1 beyond, where throughput does).  The
+ *                   automatic launch of at most one item per SM, the lowest
+ *                   end of the 4-warp range and reported as such, runs eight
+ *                   warps per item
  *   ctas_per_sm     resident CTAs per SM for that size (1..32; 0 = 32
  *                   resident warps per SM, the register limit)
- *   smem_plates     plates of each item kept in shared memory (0..8, the
- *                   rest in the global pool; -1 = as many as fit, at most 4)
+ *   smem_plates     plates of each item whose cells are kept in shared
+ *                   memory (0..8, the rest in the global pool; -1 = none, and
+ *                   as many plates per CTA as would fit, at most 4, besides
+ *                   the pool)
  *   task_max        0..8192, -1 = the default 8192: a warp that tests 32
  *                   candidate rows deals the (candidate that passed the
- *                   vacancy filter, 32-column output word) pairs across its
- *                   lanes when there are at most task_max of them, else each
- *                   lane tests its own candidate
+ *                   vacancy filter, 64 columns) pairs across its lanes when
+ *                   there are at most task_max of them, else each lane tests
+ *                   its own candidate
  * ctas_per_sm and smem_plates need an explicit warps_per_item (with 0 they
  * must be 0 and -1).  A shape that cannot be resident is refused with
  * BRKGA_ERR_INVALID_ARGUMENT and the previous configuration kept.  The
