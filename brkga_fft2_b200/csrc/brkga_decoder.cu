@@ -20,7 +20,7 @@
 //      gene) 64-bit keys in shared memory -> per-(chromosome, machine) part
 //      order (placement.py:118-135).  order_items_kernel then sorts the
 //      (chromosome, machine) items of all instances by part count.
-//   2. decode_kernel       persistent CTAs of 1, 2 or 4 warps (the launch
+//   2. decode_kernel       persistent CTAs of 1, 2, 4 or 8 warps (the launch
 //      shape), one (chromosome, machine) item at a time, longest first, from
 //      a device counter.  A plate is a grid of L rows of ceil(W/32)+2 32-bit
 //      words (bit x of a row = cell x) and the coarse data derived from it
@@ -100,22 +100,20 @@ struct CoarseIdx {
 
 // The rotations of one part type that fit one machine's plate
 // (numba_utils.py:82-84), fixed per (type, machine) and so built once at
-// problem creation: in rotation order and by height (stable; the order of
-// CTAs with fewer than four warps), the smallest height, and the words one
+// problem creation: by height, the smallest height, and the words one
 // read of the plate and of each rotated mask takes (the scan-bytes counter).
 struct RotList {
   unsigned char nr;
-  unsigned char r[4];   // rotation order
   unsigned char rs[4];  // by height, ties in rotation order
   unsigned char pad[3];
   int hmin;
   unsigned int scan_words;
 };
-static_assert(sizeof(RotList) == 20, "RotList layout");
+static_assert(sizeof(RotList) == 16, "RotList layout");
 
 struct MachDev {
   int L, W, NW, RS;  // plate rows, columns, words per row, row stride (NW + 2 zero pad words)
-  int NB, PS;        // blocks of rows, words of one erosion plane (NB * RS)
+  int NB;            // blocks of rows
   double area;       // MachineData.bin_area
   double setup;      // MachineData.setup_time
 };
@@ -148,7 +146,7 @@ struct Tables {
   const int32_t* best_rot;
   const RotDev* rot;        // [absolute type * 4 + rotation]
   const CoarseIdx* cidx;    // [rotation, indexed like rot][offset of the top row in a block]
-  const uint2* centry;      // (first column | second window's offset << 16, block row | plane << 16)
+  const uint2* centry;      // (first window's column | second one's << 16, plane row from the top row's block on)
   const uint32_t* cfilter;
   const uint2* truns;       // (start | length << 16, row) per run of ones
   const uint2* tsegs;       // the same, lengths at most 32
@@ -189,7 +187,7 @@ struct Run {
   int crit_items;      // items at the head of the queue that mark their SM (0 = off)
   unsigned long long* counters;
   BinScal* binscal;  // Nmax per resident CTA
-  uint32_t* pool;    // grids of the plates that are not in shared memory, grid_words each
+  uint32_t* pool;    // grids of the plates beyond the CTAs' own, grid_words each
   uint32_t* cpool;   // their erosion planes and block vacancies, coarse_words each
   long long pool_bins;
   uint32_t* own;     // S plates per resident CTA, grid and planes
@@ -307,7 +305,7 @@ constexpr int kGroupSegs = 4;  // this many pieces of each
 // Where one open plate lives.
 struct PlateRef {
   uint32_t* grid;    // L rows of RS words
-  uint32_t* planes;  // n_planes x NB rows of RS words
+  uint32_t* planes;  // NB x n_planes rows of RS words
   uint16_t* vac;     // NB longest free runs
 };
 
@@ -339,10 +337,11 @@ __device__ __forceinline__ PlateRef plate_ref(const Run& run, uint32_t* smem, in
 // pairs that pass the filter at P100M4, one in ten stays open.  What bounds the
 // kernel is integer issue on chip, so the instructions of a rejected position
 // are what counts: before, lanes walked the runs of its rows, some fifty
-// instructions for each run and 32 columns.  One launch before / now: P100M4 1.54 / 1.08 ms (500 rows) and 8.25 / 5.8 ms (4,000),
-// P200M6 3.94 / 2.58 ms (1,000), P400M8 35.9 / 19.8 ms (1,024), P50M2 0.404 /
-// 0.307 ms (1 row) and 0.523 / 0.392 ms (100), 64 uneven instances x 256
-// 29.5 / 21.1 ms.
+// instructions for each run and 32 columns.  One launch
+// before / now: P100M4 1.54 / 1.04 ms (500 rows) and 8.25 / 5.47 ms (4,000),
+// P200M6 3.94 / 2.45 ms (1,000), P400M8 35.9 / 18.65 ms (1,024), P50M2 0.404 /
+// 0.252 ms (1 row) and 0.523 / 0.355 ms (100), 64 uneven instances x 256
+// 29.5 / 19.8 ms.
 //
 // The filter: every block has a free run as long as the core it must take.
 __device__ __forceinline__ bool coarse_ok(const Tables& tb, const uint16_t* vac, int ty, int rot) {
@@ -361,13 +360,17 @@ __device__ __forceinline__ bool coarse_ok(const Tables& tb, const uint16_t* vac,
   return true;
 }
 
-// Columns base .. base + 63 at which one core is free: its run is the union of
-// two windows of the plane's length (the entry's plane is the longest that
-// fits; longer cores are several entries).
-__device__ __forceinline__ uint2 coarse_window(const uint32_t* pl, const MachDev& md, int base, uint2 e) {
-  const uint32_t* row = pl + (e.y & 0xFFFFu) * md.RS + (e.y >> 16) * md.PS;
-  const int p = base + (int)(e.x & 0xFFFFu), q = p + (int)(e.x >> 16);
-  const uint32_t *u = row + (p >> 5), *v = row + (q >> 5);
+// The 64 columns from pl's word on at which one core is free: its run is the
+// union of two windows of the plane's length (the entry's plane is the longest
+// that fits; longer cores are several entries).  The planes of a block lie row
+// after row and the entry holds both windows' columns, so an address is one
+// multiplication and no sum (with the planes one after another and the second
+// window as an offset, six instructions more a core): P100M4 4,000 rows 5.67 ->
+// 5.47 ms, P200M6 1,000 2.53 -> 2.45, P400M8 1,024 19.7 -> 18.65, P50M2 1 row
+// 0.257 -> 0.252.
+__device__ __forceinline__ uint2 coarse_window(const uint32_t* pl, unsigned RS, uint2 e) {
+  const uint32_t *u = pl + e.y * RS + ((e.x & 0xFFFFu) >> 5), *v = pl + e.y * RS + (e.x >> 21);
+  const uint32_t p = e.x, q = e.x >> 16;  // the shifts take their low five bits
   const uint32_t u1 = u[1], v1 = v[1];
   return make_uint2(__funnelshift_r(u[0], u1, p) & __funnelshift_r(v[0], v1, q),
                     __funnelshift_r(u1, u[2], p) & __funnelshift_r(v1, v[2], q));
@@ -377,11 +380,11 @@ __device__ __forceinline__ uint2 coarse_window(const uint32_t* pl, const MachDev
 __device__ __forceinline__ uint2 coarse_and(const Tables& tb, const uint32_t* planes, const MachDev& md, int ty, int base,
                                             uint2 F, int rot) {
   const CoarseIdx ci = tb.cidx[(rot << tb.bsh) + (ty & ((1 << tb.bsh) - 1))];
-  const uint2* c = tb.centry + ci.e;
-  const uint32_t* pl = planes + (ty >> tb.bsh) * md.RS;
-  for (int q = 0; q < ci.ne && (F.x | F.y); q += 2) {
-    const uint2 e0 = __ldg(c + q), e1 = __ldg(c + q + 1);
-    const uint2 a = coarse_window(pl, md, base, e0), b = coarse_window(pl, md, base, e1);
+  const uint4* c = reinterpret_cast<const uint4*>(tb.centry + ci.e);  // e and ne are even
+  const uint32_t* pl = planes + (ty >> tb.bsh) * tb.n_planes * md.RS + (base >> 5);
+  for (int q = 0; 2 * q < ci.ne && (F.x | F.y); ++q) {
+    const uint4 e = __ldg(c + q);
+    const uint2 a = coarse_window(pl, md.RS, make_uint2(e.x, e.y)), b = coarse_window(pl, md.RS, make_uint2(e.z, e.w));
     F.x &= a.x & b.x;
     F.y &= a.y & b.y;
   }
@@ -835,7 +838,7 @@ __device__ __forceinline__ void update_blocks(const Tables& tb, const MachDev& m
     for (int w0 = 0; w0 < md.NW; w0 += step) {
       const int w = w0 + gl;
       const uint32_t e0 = on && w < md.NW ? block_free(row, md, rows, w) : 0u;
-      uint32_t* dst = pr.planes + (size_t)b * md.RS + w;
+      uint32_t* dst = pr.planes + (size_t)b * tb.n_planes * md.RS + w;
       const bool put = on && w < md.NW && gl < step;
       uint32_t e = e0;
 #pragma unroll
@@ -844,7 +847,7 @@ __device__ __forceinline__ void update_blocks(const Tables& tb, const MachDev& m
         uint32_t nx = __shfl_down_sync(kFull, e, 1, G);
         if (gl + 1 >= G) nx = 0u;
         e &= __funnelshift_r(e, nx, 1 << (k - 1));
-        if (k >= kPlaneMin && put) dst[(size_t)(k - kPlaneMin) * md.PS] = e;
+        if (k >= kPlaneMin && put) dst[(k - kPlaneMin) * md.RS] = e;
       }
       if (md.NW <= 32) {
         // longest run of set bits over the group's words: inside a word, or
@@ -944,14 +947,19 @@ __device__ __forceinline__ void open_plate(const Tables& tb, const MachDev& md, 
   const int tid = threadIdx.x;
   if (cells) {
     for (int i = tid; i < md.L * md.RS; i += blockDim.x) pr.grid[i] = 0u;
-    const int step = (int)blockDim.x % md.RS;
-    for (int i = tid, w = tid % md.RS; i < md.PS; i += blockDim.x) {  // w: the word's place in its row
+    const int dw = (int)blockDim.x % md.RS, db = (int)blockDim.x / md.RS;
+    for (int b = tid / md.RS, w = tid % md.RS; b < md.NB;) {  // w: the word's place in its row
+      uint32_t* dst = pr.planes + (size_t)b * tb.n_planes * md.RS + w;
       for (int p = 0; p < tb.n_planes; ++p) {
         const int n = md.W - (1 << (kPlaneMin + p)) + 1 - 32 * w;  // run starts from this word on
-        pr.planes[(size_t)p * md.PS + i] = n <= 0 ? 0u : n >= 32 ? kFull : (1u << n) - 1u;
+        dst[p * md.RS] = n <= 0 ? 0u : n >= 32 ? kFull : (1u << n) - 1u;
       }
-      w += step;
-      if (w >= md.RS) w -= md.RS;
+      b += db;
+      w += dw;
+      if (w >= md.RS) {
+        w -= md.RS;
+        ++b;
+      }
     }
     for (int i = tid; i < md.NB; i += blockDim.x) pr.vac[i] = (uint16_t)md.W;
   }
@@ -990,7 +998,7 @@ struct ItemCtx {
 
 // The tables go by value (every access has a fixed parameter offset); only
 // the per-launch instance array, which is searched, is a grid constant.
-// kThreads = 32, 64 or 128 (1, 2 or 4 warps per item); 32 resident warps
+// kThreads = 32, 64, 128 or 256 (1, 2, 4 or 8 warps per item); 32 resident warps
 // per SM cap the kernel at 64 registers, which it fits without spilling.
 // Launches that leave the GPU's SMs with a few items each are bound by one
 // item's chain of instructions instead: kRoomyCtas CTAs of 128 threads per SM
@@ -1195,10 +1203,11 @@ __global__ void reduce_kernel(const __grid_constant__ Tables tb, const __grid_co
 // one (the keys of alternate parts have buffers of their own, so none is
 // overwritten before every CTA has read it).  What bounds it is the latency of
 // one search and one insertion per part: the call took 7.4 ms on one CTA of
-// four warps and takes 2.4 ms here at 100 parts on four machines (P100M4),
-// 17.4 and 4.9 ms at 200 parts on six (P200M6), 1.34 and 0.94 ms at 50 parts
-// on two (P50M2); with four warps per CTA 2.9, 5.5 and 1.05 ms, with sixteen
-// 2.35, 4.9 and 0.93 ms.
+// four warps with the search of runs and takes 1.65 ms here at 100 parts on four
+// machines (P100M4), 17.4 and 3.0 ms at 200 parts on six (P200M6), 1.34 and 0.70
+// ms at 50 parts on two (P50M2).  Before the erosion planes, with four / eight /
+// sixteen warps per CTA: 2.9 / 2.4 / 2.35 ms, 5.5 / 4.9 / 4.9 and 1.05 / 0.94 /
+// 0.93 ms.
 // Single-instance problems only, so every table base is 0.
 struct GreedyArgs {
   int N, M, T;
@@ -1700,7 +1709,7 @@ int configure(BrkgaProblem* pb, int warps_req, int ctas_req, int plates_req) {
     NBmax = std::max(NBmax, m.NB);
     Lmax = std::max(Lmax, m.L);
     grid = std::max(grid, m.L * m.RS);
-    planes = std::max(planes, pb->tb.n_planes * m.PS);
+    planes = std::max(planes, pb->tb.n_planes * m.NB * m.RS);
   }
   const int grid_words = (int)align_up((size_t)grid, 4);
   const int coarse_words = (int)align_up((size_t)planes + (size_t)(NBmax + 1) / 2, 4);
@@ -1925,7 +1934,7 @@ void coarse_tables(const std::vector<std::pair<int, int>>& longest, const RotDev
           len = 1 << kPlaneMin;
         }
         while (p < kPlaneMax && (2 << p) <= len) ++p;
-        g.centry.push_back(make_uint2((uint32_t)(k.lo + at) | ((uint32_t)(len - (1 << p)) << 16),
+        g.centry.push_back(make_uint2((uint32_t)(k.lo + at) | ((uint32_t)(k.lo + at + len - (1 << p)) << 16),
                                       (uint32_t)k.block | ((uint32_t)(p - kPlaneMin) << 16)));
         g.n_planes = std::max(g.n_planes, p - kPlaneMin + 1);
         at += len;
@@ -2064,7 +2073,6 @@ void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
     md.NW = (md.W + 31) / 32;
     md.RS = md.NW + 2;
     md.NB = (md.L + (1 << g.bsh) - 1) >> g.bsh;
-    md.PS = md.NB * md.RS;
     md.area = d->bin_area[m];
     md.setup = d->setup_time[m];
     g.mach.push_back(md);
@@ -2088,7 +2096,7 @@ void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
         const int h = d->rot_h[t * 4 + r], w = d->rot_w[t * 4 + r];
         if (h <= md.L && w <= md.W) {  // numba_utils.py:82-84
           rh[l.nr] = h;
-          l.r[l.nr] = l.rs[l.nr] = (unsigned char)r;
+          l.rs[l.nr] = (unsigned char)r;
           ++l.nr;
           l.hmin = std::min(l.hmin, h);
           l.scan_words += (unsigned)(md.L * md.NW + h * ((w + 31) / 32));
@@ -2286,6 +2294,7 @@ int brkga_problem_create_multi(const BrkgaProblemDesc* descs, int32_t K, BrkgaPr
   Merged g;
   g.bsh = block_shift(descs, K);
   for (int k = 0; k < K; ++k) merge_instance(&descs[k], g);
+  for (uint2& e : g.centry) e.y = (e.y & 0xFFFFu) * (uint32_t)g.n_planes + (e.y >> 16);  // the number of planes is known now
   if (g.maskbits.size() >= ((size_t)1 << 31) || g.truns.size() >= ((size_t)1 << 31) ||
       g.centry.size() >= ((size_t)1 << 31))
     return BRKGA_ERR_BAD_INSTANCE;
