@@ -4,15 +4,16 @@ The decode kernel has four knobs (``brkga_set_launch_config``).  Warps per
 item (1, 2 or 4) trade the latency of one (chromosome, machine) item against
 throughput: 4 finish an item sooner, 2 waste fewer lanes on speculative row
 chunks, so 2 win once the items fill several waves of resident CTAs, and 1
-(no CTA barrier at all) wins by a few per cent only when they fill some 20
-waves (measured: 64 uneven instances x 256 chromosomes, 52,000 items, 33.0
-against 35.4 ms); the automatic choice follows these tiers.  More
-resident CTAs per SM hide more latency, more plates per item in shared
-memory keep more collision searches off the global pool, and both draw on
-the same 228 KB of shared memory per SM, whose share per plate grows with
-the plate grid (a 500 x 500 plate is 36 KB as bit-packed rows, a 150 x 150
-one 3.6 KB).  The fourth, ``task_max``, decides when a warp
-deals (candidate row, 32-column word) pairs of the exact collision test
+(no CTA barrier at all) wins by 3 to 8 per cent once they fill some seven waves
+of 2-warp CTAs; the automatic choice follows these tiers (1 only from sixteen
+waves on, and 8 for a launch of at most one item per SM, which no explicit shape
+does).  More
+resident CTAs per SM hide more latency, plate grids in shared memory spare L1
+and L2 some of the searches' reads, and both draw on the same 228 KB of shared
+memory per SM, whose share per plate grows with the plate grid (a 500 x 500
+plate is 36 KB as bit-packed rows, a 150 x 150 one 4.2 KB); the automatic choice
+keeps the grids in the workspace.  The fourth, ``task_max``, decides when a warp
+deals (candidate row, 64 candidate columns) pairs of the collision test
 across its lanes instead of giving each lane one candidate row: dealing wins
 while the pairs are few, loses on wide plates with many surviving candidates
 (long, uneven chains), so its best value depends on the grid and masks.
