@@ -89,6 +89,7 @@ struct RotDev {
   int trun, ntrun;   // runs of ones of all rows in test order: truns[trun .. trun + ntrun)
   int tseg, ntseg;   // the same runs in pieces of at most 32 columns: tsegs[tseg .. tseg + ntseg)
   int mask_base;     // first word in maskbits[] (h * mw words)
+  int gseg;          // pieces that groups of lanes test first (0: none, see group_segs())
 };
 
 // The coarse test of one rotation at one alignment (its entries in centry[]
@@ -154,8 +155,8 @@ struct Tables {
   const uint8_t* newbin_ok;
   const uint8_t* fits;
   const RotList* rl;        // [(type, machine)], indexed like fits
-  int bsh;                  // a block of the coarse test has 2^bsh rows
-  int n_planes;             // erosion plane i holds the starts of free runs of 2^(kPlaneMin + i) columns
+  int bsh;                  // a block of the coarse test has 2^bsh rows (0: the test is by rows, see coarse_blocks())
+  int n_planes;             // erosion plane i holds the starts of free runs of 2^(kPlaneMin + i) columns; by rows none
 };
 
 // One instance's slice of a launch.
@@ -300,7 +301,7 @@ __device__ __forceinline__ uint2 blocked64(const uint32_t* row, int p0, int d, i
 constexpr int kTestIlp = 2;   // independent run dilations per step of the exact test
 constexpr int kVacIlp = 2;    // block vacancies compared per step of the filter
 constexpr int kGroupOpen = 3;  // pairs open after the coarse test from which groups of lanes first test
-constexpr int kGroupSegs = 4;  // this many pieces of each
+constexpr int kGroupSegs = 4;  // this many pieces of each (where the test is by rows: see group_segs())
 
 // Where one open plate lives.
 struct PlateRef {
@@ -467,6 +468,25 @@ __device__ __forceinline__ uint32_t block_free(const uint32_t* row, int RS, int 
   const int valid = W - 32 * w;
   if (valid < 32) v |= 0xFFFFFFFFu << valid;
   return ~v;
+}
+
+// longest run of free columns of one plate row (one thread)
+__device__ __forceinline__ int row_free_run(const uint32_t* row, const MachDev& md) {
+  int run = 0, best = 0;
+  for (int w = 0; w < md.NW; ++w) {
+    const uint32_t v = ~block_free(row, md.RS, md.W, 1, w);
+    if (v == 0u) {
+      run += 32;
+      continue;
+    }
+    const int tz = __ffs(v) - 1;
+    run += tz;
+    best = max(best, run);
+    const int hb = 31 - __clz(v);
+    if (hb > tz + 1) best = max(best, longest_ones(~v & ((1u << hb) - 1u) & ~((2u << tz) - 1u)));
+    run = __clz(v);
+  }
+  return max(best, run);
 }
 
 // longest run of free columns of a block of plate rows (plates wider than
@@ -648,7 +668,7 @@ struct SearchShared {
 // skip chunks that cannot beat the best key found so far, stop once no
 // rotation can at the current level, and merge with atomicMin.  Called by
 // all threads of the CTA; contains __syncthreads.
-template <int kWarps>
+template <bool kPlain, int kWarps>
 __device__ __forceinline__ unsigned long long search_plate(const Tables& tb, const MachDev& md,
                                                            const PlateRef& pr, int enc,
                                                            int t, const RotList* rlp, int task_max, int32_t* status,
@@ -742,7 +762,7 @@ __device__ __forceinline__ unsigned long long search_plate(const Tables& tb, con
     __syncwarp();
     const unsigned inv = sh.inv[slot];
     const uint2* segs = tb.tsegs + sh.rd[slot].tseg;
-    const int nseg = sh.rd[slot].ntseg;
+    const int nseg = sh.rd[slot].ntseg, gseg = kPlain ? kGroupSegs : sh.rd[slot].gseg;
     bool won = false;
     for (int t0 = 0; t0 < ntask && !won; t0 += 32) {
       // ---- the round's first pair has the smallest key left in the chunk: stop when it cannot win
@@ -765,16 +785,20 @@ __device__ __forceinline__ unsigned long long search_plate(const Tables& tb, con
       const int n_open = __popc(open), pk = row0 << 13 | base;
       int q0 = 0;
       // ---- several pairs open: 32 / 2^lg of them at once, 2^lg lanes each
-      if (n_open >= kGroupOpen) {
+      if (n_open >= kGroupOpen && gseg) {
         const int lg = n_open <= 4 ? 3 : n_open <= 8 ? 2 : n_open <= 16 ? 1 : 0;
         unsigned m = open;
-        for (int k = 0; k < (32 >> lg) - 1; ++k)
-          if (k < lane >> lg) m &= m - 1u;  // drop the pairs of the groups below
+        if (lg) {
+          for (int k = 0; k < (32 >> lg) - 1; ++k)
+            if (k < lane >> lg) m &= m - 1u;  // drop the pairs of the groups below
+        } else {
+          m &= 1u << lane;  // a lane each: its own
+        }
         const int src = m ? __ffs(m) - 1 : 0;
         const int pl = __shfl_sync(kFull, pk, src);
         uint32_t lo = __shfl_sync(kFull, F.x, src), hi = __shfl_sync(kFull, F.y, src);
         if (!m) lo = hi = 0u;
-        const int basel = pl & 0x1FFF, n = min(max(kGroupSegs, 1 << lg), nseg);
+        const int basel = pl & 0x1FFF, n = min(max(gseg, 1 << lg), nseg);
         const uint32_t* g0 = pr.grid + (size_t)(pl >> 13) * md.RS;
         for (int q = lane & ((1 << lg) - 1); q < n && (lo | hi); q += 1 << lg) {
           const uint2 e = __ldg(segs + q);
@@ -787,11 +811,12 @@ __device__ __forceinline__ unsigned long long search_plate(const Tables& tb, con
           lo &= __shfl_xor_sync(kFull, lo, o);
           hi &= __shfl_xor_sync(kFull, hi, o);
         }
-        const int from = __popc(open & ((1u << lane) - 1u)) << lg;  // this lane's pair was the group's at `from`
+        // this lane's pair was the group's at `from`
+        const int from = lg ? __popc(open & ((1u << lane) - 1u)) << lg : lane;
         F.x &= __shfl_sync(kFull, lo, from & 31);
         F.y &= __shfl_sync(kFull, hi, from & 31);
         open &= __ballot_sync(kFull, (F.x | F.y) != 0u);
-        q0 = max(kGroupSegs, 1 << lg);
+        q0 = max(gseg, 1 << lg);
       }
       // ---- exact test of the open pairs in order
       while (open) {
@@ -830,12 +855,13 @@ __device__ __forceinline__ unsigned long long search_plate(const Tables& tb, con
 // rows.  A group of 8, 16 or 32 lanes takes a block, a lane one word of it (on
 // plates wider than 1024 columns a warp walks the row in steps that overlap by
 // the words an erosion reaches).  All threads of the CTA; no barrier.
+template <bool kPlain>
 __device__ __forceinline__ void update_blocks(const Tables& tb, const MachDev& md, const PlateRef& pr, int b0, int b1) {
   const int lane = threadIdx.x & 31;
   const int G = md.NW <= 8 ? 8 : md.NW <= 16 ? 16 : 32, gl = lane & (G - 1);
   const int groups = blockDim.x / G;
   constexpr int kReach = (1 << kPlaneMax) / 32 + 1;  // words past its own that a plane word depends on
-  const int step = md.NW <= 32 ? 32 : 32 - kReach;
+  const int step = kPlain || md.NW <= 32 ? 32 : 32 - kReach;
   for (int bb = b0; bb <= b1; bb += groups) {
     const int b = bb + (int)threadIdx.x / G;
     const bool on = b <= b1;
@@ -855,7 +881,7 @@ __device__ __forceinline__ void update_blocks(const Tables& tb, const MachDev& m
         e &= __funnelshift_r(e, nx, 1 << (k - 1));
         if (k >= kPlaneMin && put) dst[(k - kPlaneMin) * md.RS] = e;
       }
-      if (md.NW <= 32) {
+      if (kPlain || md.NW <= 32) {
         // longest run of set bits over the group's words: inside a word, or
         // from a word's top bits through full words into the next one's low bits
         const unsigned fm = __ballot_sync(kFull, e0 == kFull) >> (lane - gl);
@@ -870,7 +896,7 @@ __device__ __forceinline__ void update_blocks(const Tables& tb, const MachDev& m
         if (on && gl == 0) pr.vac[b] = (uint16_t)run;
       }
     }
-    if (md.NW > 32 && on) {  // the group is the warp
+    if (!kPlain && md.NW > 32 && on) {  // the group is the warp
       const int run = max_free_run(row, md.RS, md.W, md.NW, rows);
       if (gl == 0) pr.vac[b] = (uint16_t)run;
     }
@@ -903,16 +929,18 @@ __device__ __forceinline__ void or_row(uint32_t* dst, const uint32_t* m, int mw,
 
 // Insert rotation r of part type t (absolute) with its top row at ty and left
 // column x (binClassNew.py:155-174): OR the mask rows into the plate words,
-// then recompute the touched blocks' planes and vacancies; thread 0 updates
-// the plate scalars with the part's area and times on this machine.  Without
+// then recompute the touched blocks' planes and vacancies (where the test is by
+// rows, the row's vacancy with the row); thread 0 updates the plate scalars with the part's area and times on this machine.  Without
 // `cells` (no search of the item follows) only the scalars.
 // All threads of the CTA; ends with __syncthreads.
+template <bool kPlain>
 __device__ __forceinline__ void place_part(const Tables& tb, const MachDev& md, const PlateRef& pr, BinScal* scal, int t,
                                            int r, int x, int ty, double a, double ptv, double pthv, bool cells) {
   const int tid = threadIdx.x;
   const RotDev rd = tb.rot[t * 4 + r];
   const int sx = x & 31, wx = x >> 5, mw = rd.mw;
   const uint32_t* mb = tb.maskbits + rd.mask_base;
+  const bool by_rows = !kPlain && tb.bsh == 0;
   for (int i = tid; i < rd.h && cells; i += blockDim.x) {
     uint32_t* row = pr.grid + (size_t)(ty + i) * md.RS;
     const uint32_t* m = mb + (size_t)i * mw;
@@ -932,6 +960,7 @@ __device__ __forceinline__ void place_part(const Tables& tb, const MachDev& md, 
       const uint32_t v = __funnelshift_l(prev, 0u, sx);
       if (v) dst[mw] |= v;
     }
+    if (by_rows) pr.vac[ty + i] = (uint16_t)row_free_run(row, md);
   }
   if (tid == 0) {
     BinScal s = *scal;
@@ -944,20 +973,21 @@ __device__ __forceinline__ void place_part(const Tables& tb, const MachDev& md, 
     *scal = s;
   }
   __syncthreads();
-  if (!cells) return;
-  update_blocks(tb, md, pr, ty >> tb.bsh, (ty + rd.h - 1) >> tb.bsh);
+  if (!cells || by_rows) return;
+  update_blocks<kPlain>(tb, md, pr, ty >> tb.bsh, (ty + rd.h - 1) >> tb.bsh);
   __syncthreads();
 }
 
 // Empty plate: zero words, every run of columns free (binClassNew.py:18-20),
 // fresh scalars.  Without `cells` only the scalars.
+template <bool kPlain>
 __device__ __forceinline__ void open_plate(const Tables& tb, const MachDev& md, const PlateRef& pr, BinScal* scal,
                                            int pool_index, bool cells) {
   const int tid = threadIdx.x;
   if (cells) {
     for (int i = tid; i < md.L * md.RS; i += blockDim.x) pr.grid[i] = 0u;
     const int dw = (int)blockDim.x % md.RS, db = (int)blockDim.x / md.RS;
-    for (int b = tid / md.RS, w = tid % md.RS; b < md.NB;) {  // w: the word's place in its row
+    for (int b = tid / md.RS, w = tid % md.RS; b < md.NB && (kPlain || tb.n_planes);) {  // w: the word's place in its row
       uint32_t* dst = pr.planes + (size_t)b * tb.n_planes * md.RS + w;
       for (int p = 0; p < tb.n_planes; ++p) {
         const int n = md.W - (1 << (kPlaneMin + p)) + 1 - 32 * w;  // run starts from this word on
@@ -1018,7 +1048,10 @@ struct ItemCtx {
 // 80 rows 0.77 / 0.66 / -; with 200 items on 148 SMs eight warps gain 2 % (P50M2)
 // or lose 5 % (246 small parts).
 constexpr int kRoomyCtas = 4;
-template <int kThreads, int kMinCtas = kResidentWarps * 32 / kThreads>
+// kPlain: the test is by blocks and no plate is wider than 1024 columns, as in
+// most problems; without what the others need the kernel is 1 to 1.5 % faster
+// (P100M4 4,000 rows 5.49 -> 5.42 ms, 500 rows 1.02 -> 0.99).
+template <bool kPlain, int kThreads, int kMinCtas = kResidentWarps * 32 / kThreads>
 __global__ void __launch_bounds__(kThreads, kMinCtas)
     decode_kernel(const Tables tb, const __grid_constant__ Run run) {
   extern __shared__ __align__(16) uint32_t smem[];
@@ -1105,7 +1138,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas)
       for (int b = 0; b < nb; ++b) {
         if (bs[b].area + a > md.area) continue;  // placement.py:57-59
         const PlateRef pr = plate_ref(run, smem, b, bs[b].pool);
-        key = search_plate(tb, md, pr, bs[b].enc, t,
+        key = search_plate<kPlain>(tb, md, pr, bs[b].enc, t,
                            tb.rl + ctx.tmbase + (size_t)(t - ctx.tbase) * ctx.M + ctx.m, run.task_max, run.status,
                            sh2[sh_par], c_tests, c_chunks, c_bytes);
         sh_par ^= 1;
@@ -1143,7 +1176,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas)
         }
         pb = nb++;
         owned = max(owned, nb - run.S);
-        open_plate(tb, md, plate_ref(run, smem, pb, s_pool), &bs[pb], s_pool, !last);
+        open_plate<kPlain>(tb, md, plate_ref(run, smem, pb, s_pool), &bs[pb], s_pool, !last);
         if (tid == 0) ++c_bins;
         x = 0;
         ty = md.L - tb.rot[t * 4 + r].h;
@@ -1155,7 +1188,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas)
 
       // ---- insert (binClassNew.py:155-174)
       const size_t tm = (size_t)ctx.tmbase + (size_t)ctx.m * ctx.T + (t - ctx.tbase);
-      place_part(tb, md, plate_ref(run, smem, pb, bs[pb].pool), &bs[pb], t, r, x, ty, a, tb.pt[tm], tb.pth[tm], !last);
+      place_part<kPlain>(tb, md, plate_ref(run, smem, pb, bs[pb].pool), &bs[pb], t, r, x, ty, a, tb.pt[tm], tb.pth[tm], !last);
       if (tid == 0 && lg) lg[k] = BrkgaPlacement{gene, pb, x, ty + tb.rot[t * 4 + r].h - 1, r};
     }
     if (!failed && tid == 0) {  // placement.py:86-89
@@ -1265,7 +1298,7 @@ __device__ __forceinline__ void cluster_store(unsigned long long* p, unsigned ra
                : "memory");
 }
 
-__global__ void __launch_bounds__(kGreedyThreads) greedy_kernel(const __grid_constant__ Tables tb,
+__global__ void __launch_bounds__(kGreedyThreads, 1) greedy_kernel(const __grid_constant__ Tables tb,
                                                                 const __grid_constant__ GreedyArgs g) {
   extern __shared__ __align__(16) unsigned char gsm[];
   const unsigned rank = cluster_rank();
@@ -1308,7 +1341,7 @@ __global__ void __launch_bounds__(kGreedyThreads) greedy_kernel(const __grid_con
       unsigned long long key = kKeyNone;
       if (tb.fits[t * g.M + m]) {  // BRKGA_alg3.py:465-470
         const PlateRef pr = greedy_plate(g, b);
-        key = search_plate(tb, md, pr, bs[b].enc, t,
+        key = search_plate<false>(tb, md, pr, bs[b].enc, t,
                            tb.rl + (size_t)t * g.M + m, kDefaultTaskMax, g.status, sh2[sh_par], c_tests, c_chunks,
                            c_bytes);
         sh_par ^= 1;
@@ -1391,8 +1424,8 @@ __global__ void __launch_bounds__(kGreedyThreads) greedy_kernel(const __grid_con
     cw = cw > c.cand ? cw : c.cand;
     if ((unsigned)b % kGreedyCtas == rank) {
       const PlateRef pr = greedy_plate(g, b);
-      if (fresh) open_plate(tb, md, pr, &bs[b], c.machine, true);
-      place_part(tb, md, pr, &bs[b], t, r, x, ty, a, tb.pt[(size_t)c.machine * g.T + t],
+      if (fresh) open_plate<false>(tb, md, pr, &bs[b], c.machine, true);
+      place_part<false>(tb, md, pr, &bs[b], t, r, x, ty, a, tb.pt[(size_t)c.machine * g.T + t],
                  tb.pth[(size_t)c.machine * g.T + t], true);
       if (tid == 0) {
         g.out_machine[k] = c.machine;
@@ -1526,6 +1559,7 @@ struct BrkgaProblem {
   int sm_count = 0;
   int req_warps = 0, req_ctas = 0, req_plates = -1;  // requested launch shape (0 / 0 / -1 = automatic)
   int task_max = kDefaultTaskMax;
+  bool plain = false;  // the kernels' plain forms serve (see decode_kernel)
   Shape shape[3];      // 4, 2 and 1 warps per item
   int min_S = 0;       // fewest own plates per CTA of the three shapes (pool sizing)
   int grid_words = 0, coarse_words = 0, vac_off = 0;  // words of a plate's grid, of its planes and vacancies, of the planes
@@ -1681,20 +1715,34 @@ class DeviceGuard {
   int prev_ = 0;
 };
 
-template <int kThreads, int kMinCtas = kResidentWarps * 32 / kThreads>
-int prepare_kernel(size_t dyn_max) {
-  return cudaFuncSetAttribute(decode_kernel<kThreads, kMinCtas>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_max) ==
-                 cudaSuccess
+// The forms of the decode kernel: warps per item, and with 128 registers for
+// launches of few items (kRoomyCtas).
+enum Form { kForm1, kForm2, kForm4, kForm4Roomy, kForm8, kForms };
+using DecodeKernel = void (*)(const Tables, const Run);
+template <bool kPlain>
+DecodeKernel decode_form(Form f) {
+  return f == kForm1        ? decode_kernel<kPlain, 32>
+         : f == kForm2      ? decode_kernel<kPlain, 64>
+         : f == kForm4      ? decode_kernel<kPlain, 128>
+         : f == kForm4Roomy ? decode_kernel<kPlain, 128, kRoomyCtas>
+                            : decode_kernel<kPlain, 256, 2>;
+}
+
+DecodeKernel decode_form(const BrkgaProblem* pb, Form f) {
+  return pb->plain ? decode_form<true>(f) : decode_form<false>(f);
+}
+
+int prepare_kernel(const BrkgaProblem* pb, Form f, size_t dyn_max) {
+  return cudaFuncSetAttribute(decode_form(pb, f), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_max) == cudaSuccess
              ? BRKGA_OK
              : BRKGA_ERR_CUDA;
 }
 
-int occupancy(int warps, size_t smem, int* occ) {
-  const cudaError_t e =
-      warps == 1   ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, decode_kernel<32>, 32, smem)
-      : warps == 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, decode_kernel<64>, 64, smem)
-                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, decode_kernel<128>, 128, smem);
-  return e == cudaSuccess ? BRKGA_OK : BRKGA_ERR_CUDA;
+int occupancy(const BrkgaProblem* pb, int warps, size_t smem, int* occ) {
+  const Form f = warps == 1 ? kForm1 : warps == 2 ? kForm2 : kForm4;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, decode_form(pb, f), 32 * warps, smem) == cudaSuccess
+             ? BRKGA_OK
+             : BRKGA_ERR_CUDA;
 }
 
 // Launch shapes of the decode kernel, one per CTA size (4, 2 and 1 warps per
@@ -1726,9 +1774,9 @@ int configure(BrkgaProblem* pb, int warps_req, int ctas_req, int plates_req) {
   // room of a plate in shared memory: its grid and two bytes a row
   const size_t slot_bytes = align_up((size_t)grid + (size_t)(Lmax + 1) / 2, 4) * 4;
   cudaFuncAttributes fa4, fa2, fa1;
-  if (cudaFuncGetAttributes(&fa4, decode_kernel<128>) != cudaSuccess ||
-      cudaFuncGetAttributes(&fa2, decode_kernel<64>) != cudaSuccess ||
-      cudaFuncGetAttributes(&fa1, decode_kernel<32>) != cudaSuccess)
+  if (cudaFuncGetAttributes(&fa4, decode_form(pb, kForm4)) != cudaSuccess ||
+      cudaFuncGetAttributes(&fa2, decode_form(pb, kForm2)) != cudaSuccess ||
+      cudaFuncGetAttributes(&fa1, decode_form(pb, kForm1)) != cudaSuccess)
     return BRKGA_ERR_CUDA;
   const size_t static_smem = std::max({fa4.sharedSizeBytes, fa2.sharedSizeBytes, fa1.sharedSizeBytes});
   const size_t per_sm = prop.sharedMemPerMultiprocessor;
@@ -1736,9 +1784,8 @@ int configure(BrkgaProblem* pb, int warps_req, int ctas_req, int plates_req) {
   const size_t reserve = 1024 + static_smem;  // per-block system reservation + static shared variables
   const int max_fit = (int)std::min<size_t>(kMaxSmemPlates, per_block_max / slot_bytes);
   int st;
-  if ((st = prepare_kernel<128>(per_block_max)) || (st = prepare_kernel<64>(per_block_max)) ||
-      (st = prepare_kernel<32>(per_block_max)) || (st = prepare_kernel<128, kRoomyCtas>(per_block_max)))
-    return st;
+  for (const Form f : {kForm4, kForm2, kForm1, kForm4Roomy})
+    if ((st = prepare_kernel(pb, f, per_block_max))) return st;
   if (cudaFuncSetAttribute(assign_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxGenes * 8) !=
       cudaSuccess)
     return BRKGA_ERR_CUDA;
@@ -1783,7 +1830,7 @@ int configure(BrkgaProblem* pb, int warps_req, int ctas_req, int plates_req) {
     if (S > max_fit) return BRKGA_ERR_INVALID_ARGUMENT;
     const size_t smem = preq > 0 ? (size_t)S * grid_bytes : 0;
     int occ = 0;
-    if ((st = occupancy(warps, smem, &occ))) return st;
+    if ((st = occupancy(pb, warps, smem, &occ))) return st;
     if (occ < 1 || (creq > 0 && occ < creq)) return BRKGA_ERR_INVALID_ARGUMENT;
     shapes[v].warps = warps;
     shapes[v].S = S;
@@ -1857,7 +1904,9 @@ struct Merged {
   std::vector<uint2> centry;
   std::vector<uint32_t> cfilter;
   std::vector<uint2> tsegs;
-  int bsh = 0, n_planes = 0;  // rows of a block (2^bsh), erosion planes that some core reads
+  int bsh = 0, n_planes = 0;  // rows of a block (2^bsh, 0: by rows), erosion planes that some core reads
+  std::vector<std::pair<int, int>> longest;  // per mask row, rotation after rotation: [first, last + 1) of its longest run
+  std::vector<int> n_runs;                   // per rotation: runs of ones of all rows
   std::vector<uint2> truns;
   std::vector<uint32_t> maskbits;
   std::vector<uint8_t> fits, newbin_ok;
@@ -1888,19 +1937,47 @@ int block_shift(const BrkgaProblemDesc* descs, int K) {
     parts += d.n_genes;
     fill += plates > 0.0 ? d.n_genes * area / plates : 0.0;
   }
+  if (height < 13.0 * parts) return 0;  // by rows, see coarse_blocks()
   return height < 28.0 * parts || (height < 50.0 * parts && fill >= 0.6 * parts) ? 2 : 3;
+}
+
+// Where the test is by rows, a rotation's filter holds this many of its rows:
+// a tall, thin mask that passes 24 of them often fails at another one (200
+// masks of 1-3 x 20-120 cells, 2,000 rows: 24 rows 2.19 ms, 64 1.85, all 1.97).
+constexpr int kFilterRows = 64;
+
+// Pieces of a mask that groups of lanes test before the whole warp takes the
+// open pairs one by one, where the test is by rows: as many as hold kGroupCells
+// cells (4 of long runs decide as much as 20 of single cells), and none for a
+// mask of so few that one step of the warp tests them all and its few pairs are
+// soon through.  Measured (cells 20 / 32 / 48): masks of noise 1.87 / 1.64 / 1.55
+// ms, parts of 5-15 cells 1.66 / 1.80 / 1.90.  (None for up to 4 / 6 / 8 / 12
+// pieces: 1-6 cell parts 2.43 / 2.09 / 2.09 / 2.09 ms, of 5-15 cells 1.59 / 1.66
+// / 1.73 / 2.03, of 5-10 cells 1.36 / 1.35 / 1.27 / 1.19.)
+constexpr int kGroupCells = 20, kGroupFewSegs = 6, kGroupMostSegs = 20;
+int group_segs(const RotDev& rd, const Merged& g) {
+  if (g.bsh) return kGroupSegs;
+  if (rd.ntseg <= kGroupFewSegs) return 0;
+  int cells = 0, q = 0;
+  for (; q < rd.ntseg && q < kGroupMostSegs && (q < kGroupSegs || cells < kGroupCells); ++q)
+    cells += (int)(g.tsegs[rd.tseg + q].x >> 16);
+  return q;
 }
 
 // The coarse test's entries of one rotation (see coarse_ok()): for every
 // offset of its top row in a block of plate rows, the blocks it covers
 // whole and the core of each, widest first, then coarse to fine from the
 // bottom (as the rows of the exact test).  Cores shorter than the first plane's
-// runs are left to the exact test.
-void coarse_tables(const std::vector<std::pair<int, int>>& longest, const RotDev& rd, Merged& g) {
+// runs are left to the exact test.  By rows every row is a block and its longest
+// run the core, for the filter only.  Returns how many of the rotation's rows are
+// part of a core, summed over the offsets.
+int coarse_tables(const std::pair<int, int>* longest, const RotDev& rd, Merged& g) {
   struct Core {
     int block, lo, len;
   };
+  const bool by_rows = g.bsh == 0;
   const int rows = 1 << g.bsh;
+  int covered = 0;
   std::vector<Core> cores;
   std::vector<int> order;
   std::vector<char> used;
@@ -1913,9 +1990,10 @@ void coarse_tables(const std::vector<std::pair<int, int>>& longest, const RotDev
         lo = std::max(lo, longest[i + k].first);
         hi = std::min(hi, longest[i + k].second);
       }
-      if (hi - lo >= (1 << kPlaneMin)) cores.push_back({(i + off) >> g.bsh, lo, hi - lo});
+      if (hi - lo >= (by_rows ? 1 : 1 << kPlaneMin)) cores.push_back({(i + off) >> g.bsh, lo, hi - lo});
     }
     const int n = (int)cores.size();
+    covered += n * rows;
     used.assign(n, 0);
     if (n) {
       int widest = 0;
@@ -1923,20 +2001,21 @@ void coarse_tables(const std::vector<std::pair<int, int>>& longest, const RotDev
         if (cores[c].len > cores[widest].len) widest = c;
       order.push_back(widest);
       used[widest] = 1;
-      for (int st = 4; st >= 1; st >>= 1)
+      for (int st = by_rows ? 16 : 4; st >= 1; st >>= 1)
         for (int c = n - 1; c >= 0; c -= st)
           if (!used[c]) {
             order.push_back(c);
             used[c] = 1;
           }
     }
+    if (by_rows && n > kFilterRows) order.resize(kFilterRows);
     CoarseIdx ci;
     ci.e = (int)g.centry.size();
     ci.f = (int)g.cfilter.size();
     for (int c : order) {
       const Core& k = cores[c];
       g.cfilter.push_back(((uint32_t)k.block << 16) | (uint32_t)k.len);
-      for (int at = 0; at < k.len;) {  // pieces of at most two windows of the longest plane
+      for (int at = 0; at < k.len && !by_rows;) {  // pieces of at most two windows of the longest plane
         int len = std::min(k.len - at, 2 << kPlaneMax), p = kPlaneMin;
         if (len < (1 << kPlaneMin)) {  // a short last piece: the first plane's window up to the core's end
           at = k.len - (1 << kPlaneMin);
@@ -1955,6 +2034,102 @@ void coarse_tables(const std::vector<std::pair<int, int>>& longest, const RotDev
     ci.nf = (int)g.cfilter.size() - ci.f;
     g.cidx.push_back(ci);
   }
+  return covered;
+}
+
+// Rotation r of type t fits the plates of some machine of its instance (the others are never tested).
+bool fits_some(const BrkgaProblemDesc& d, int t, int r) {
+  for (int m = 0; m < d.n_machines; ++m)
+    if (d.rot_h[t * 4 + r] <= d.bin_length[m] && d.rot_w[t * 4 + r] <= d.bin_width[m]) return true;
+  return false;
+}
+
+// The coarse test's tables of every rotation for blocks of 2^g.bsh rows.
+// Returns the share of the masks' rows that are part of a core, over the genes.
+double coarse_tables(const BrkgaProblemDesc* descs, int K, Merged& g) {
+  g.cidx.clear();
+  g.centry.clear();
+  g.cfilter.clear();
+  g.n_planes = 0;
+  double covered = 0.0, rows = 0.0;
+  std::vector<std::pair<double, double>> of_type;  // rows in cores, rows
+  size_t rot = 0;
+  const std::pair<int, int>* longest = g.longest.data();
+  for (int k = 0; k < K; ++k) {
+    const BrkgaProblemDesc& d = descs[k];
+    of_type.assign(d.n_types, {0.0, 0.0});
+    for (int t = 0; t < d.n_types; ++t)
+      for (int r = 0; r < 4; ++r, ++rot) {
+        if (r >= d.part_nrot[t]) {
+          g.cidx.resize(g.cidx.size() + ((size_t)1 << g.bsh), CoarseIdx{0, 0, 0, 0});
+          continue;
+        }
+        RotDev& rd = g.rot[rot];
+        const double in_cores = (double)coarse_tables(longest, rd, g) / (1 << g.bsh);
+        if (fits_some(d, t, r)) {
+          of_type[t].first += in_cores;
+          of_type[t].second += rd.h;
+        }
+        rd.gseg = group_segs(rd, g);
+        longest += rd.h;
+      }
+    for (int j = 0; j < d.n_genes; ++j) {
+      covered += of_type[d.gene_type[j]].first;
+      rows += of_type[d.gene_type[j]].second;
+    }
+  }
+  for (MachDev& m : g.mach) m.NB = (m.L + (1 << g.bsh) - 1) >> g.bsh;
+  return covered / rows;
+}
+
+// The share of the masks' rows that belong to parts with more than kMostRuns
+// runs of ones a row, over the genes.
+constexpr double kMostRuns = 2.1;
+double many_runs(const BrkgaProblemDesc* descs, int K, const Merged& g) {
+  double many = 0.0, rows = 0.0;
+  std::vector<std::pair<double, double>> of_type;  // runs, rows
+  size_t rot = 0;
+  for (int k = 0; k < K; ++k) {
+    const BrkgaProblemDesc& d = descs[k];
+    of_type.assign(d.n_types, {0.0, 0.0});
+    for (int t = 0; t < d.n_types; ++t)
+      for (int r = 0; r < 4; ++r, ++rot)
+        if (r < d.part_nrot[t] && fits_some(d, t, r)) {
+          of_type[t].first += g.n_runs[rot];
+          of_type[t].second += g.rot[rot].h;
+        }
+    for (int j = 0; j < d.n_genes; ++j) {
+      const std::pair<double, double>& p = of_type[d.gene_type[j]];
+      many += p.first > kMostRuns * p.second ? p.second : 0.0;
+      rows += p.second;
+    }
+  }
+  return many / rows;
+}
+
+// Block height and tables of the coarse test.  A block's core is one run of
+// columns, so it says little of masks whose rows have several runs (lattices,
+// plates with holes, combs) and parts of few rows have next to none; their
+// positions then went to the exact test without a filter.  Such problems are
+// tested by rows: the plate keeps the longest free run of every row instead of
+// planes, and a rotation's rows need one as long as their own longest run
+// (numba_utils.py:50-94).  By rows from a fifth of the mask rows in parts of many
+// runs on (frames, rings, H and U shapes have two runs at most), below 13 rows a
+// mask, and where less than 0.6 of the rows lie in cores at four rows a block.
+// One launch, by blocks / by rows:
+//   parts of 30-90 cells on three 300 x 300 plates, 500 rows: lattices 2.64 /
+//     0.85 ms, rectangles with holes 1.24 / 0.67, bars of 5 every 12-20 cells
+//     1.74 / 0.68; of solid parts and lattices 10 % lattices 0.79 / 0.86, 20 %
+//     1.02 / 0.89, 33 % 1.33 / 0.90; U shapes 1.18 / 1.73, frames of 4 cells
+//     0.81 / 1.27, solid parts (P100M4) 1.01 / 1.50;
+//   solid parts of 4-8 cells 1.53 / 1.20 ms, 5-15 1.92 / 1.66, 5-20 1.98 / 1.83,
+//     6-24 2.02 / 2.02, 14-25 1.08 / 1.29 (200 on three plates, 1,000 rows; the
+//     last 246 on two, 100 rows); rectangles of 4-12 cells 1.58 / 1.20, 1-3 x
+//     20-120 2.72 / 1.82 (2,000 rows).
+constexpr double kManyRunsShare = 0.2, kLeastCovered = 0.6;
+void coarse_blocks(const BrkgaProblemDesc* descs, int K, Merged& g) {
+  g.bsh = many_runs(descs, K, g) > kManyRunsShare ? 0 : block_shift(descs, K);
+  while (coarse_tables(descs, K, g) < kLeastCovered && g.bsh) g.bsh = g.bsh == 3 ? 2 : 0;
 }
 
 // A row's cells as bits, n <= 32 of them: eight bytes at a time, as (nonzero)
@@ -1999,7 +2174,6 @@ void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
   id.tmbase = (int)g.pt.size();
   std::vector<uint32_t> runs;                // one rotation's runs of ones, row after row
   std::vector<int> row_at, order;            // where each row's runs begin; the rows in test order
-  std::vector<std::pair<int, int>> longest;  // per row: [first, last + 1) of its longest run
   std::vector<char> used;
   for (int t = 0; t < T; ++t) {
     for (int r = 0; r < 4; ++r) {
@@ -2014,18 +2188,18 @@ void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
         int imax = 0, dmax = 0;  // row with the longest run of ones and that length
         runs.clear();
         row_at.assign(1, 0);
-        longest.assign(h, {0, 0});
         for (int i = 0; i < h; ++i) {
           const uint8_t* cells = mk + (size_t)i * w;
           for (int j = 0; j < w; j += 32) g.maskbits.push_back(pack_cells(cells + j, std::min(32, w - j)));
           const uint32_t* row = g.maskbits.data() + g.maskbits.size() - rd.mw;
           int best = 0;
+          g.longest.push_back({0, 0});
           for (int j = next_cell(row, w, 0, true); j < w;) {
             const int end = next_cell(row, w, j, false);
             runs.push_back((uint32_t)j | ((uint32_t)(end - j) << 16));
             if (end - j > best) {
               best = end - j;
-              longest[i] = {j, end};
+              g.longest.back() = {j, end};
             }
             j = next_cell(row, w, end, true);
           }
@@ -2064,11 +2238,9 @@ void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
         }
         rd.ntrun = (int)g.truns.size() - rd.trun;
         rd.ntseg = (int)g.tsegs.size() - rd.tseg;
-        coarse_tables(longest, rd, g);
-      } else {
-        g.cidx.resize(g.cidx.size() + ((size_t)1 << g.bsh), CoarseIdx{0, 0, 0, 0});
       }
       g.rot.push_back(rd);
+      g.n_runs.push_back(rd.ntrun);
     }
     g.area.push_back(d->part_area[t]);
     g.nrot.push_back(d->part_nrot[t]);
@@ -2081,7 +2253,7 @@ void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
     md.W = d->bin_width[m];
     md.NW = (md.W + 31) / 32;
     md.RS = md.NW + 2;
-    md.NB = (md.L + (1 << g.bsh) - 1) >> g.bsh;
+    md.NB = 0;  // coarse_tables()
     md.area = d->bin_area[m];
     md.setup = d->setup_time[m];
     g.mach.push_back(md);
@@ -2192,11 +2364,13 @@ int launch(const BrkgaProblem* pb, int stage, const Run& run, cudaStream_t s) {
   if (stage == 0 || stage == 2) {
     const Shape& sh = pick_shape(pb, run.n_items);
     const int grid = (int)std::min<int64_t>(sh.n_slots, run.n_items);
-    if (sh.warps == 1) decode_kernel<32><<<grid, 32, sh.smem, s>>>(pb->tb, run);
-    else if (sh.warps == 2) decode_kernel<64><<<grid, 64, sh.smem, s>>>(pb->tb, run);
-    else if (!pb->req_warps && grid <= pb->sm_count) decode_kernel<256, 2><<<grid, 256, 0, s>>>(pb->tb, run);
-    else if (grid <= kRoomyCtas * pb->sm_count) decode_kernel<128, kRoomyCtas><<<grid, 128, sh.smem, s>>>(pb->tb, run);
-    else decode_kernel<128><<<grid, 128, sh.smem, s>>>(pb->tb, run);
+    const bool alone = sh.warps == 4 && !pb->req_warps && grid <= pb->sm_count;  // every item has an SM to itself
+    const Form f = sh.warps == 1                       ? kForm1
+                   : sh.warps == 2                     ? kForm2
+                   : alone                             ? kForm8
+                   : grid <= kRoomyCtas * pb->sm_count ? kForm4Roomy
+                                                       : kForm4;
+    decode_form(pb, f)<<<grid, f == kForm8 ? 256 : 32 * sh.warps, sh.smem, s>>>(pb->tb, run);
   }
   if (stage == 0 || stage == 3) reduce_kernel<<<(run.n_rows + 255) / 256, 256, 0, s>>>(pb->tb, run);
   return cudaGetLastError() == cudaSuccess ? BRKGA_OK : BRKGA_ERR_CUDA;
@@ -2301,8 +2475,8 @@ int brkga_problem_create_multi(const BrkgaProblemDesc* descs, int32_t K, BrkgaPr
     return BRKGA_ERR_NO_DEVICE;
   }
   Merged g;
-  g.bsh = block_shift(descs, K);
   for (int k = 0; k < K; ++k) merge_instance(&descs[k], g);
+  coarse_blocks(descs, K, g);
   for (uint2& e : g.centry) e.y = (e.y & 0xFFFFu) * (uint32_t)g.n_planes + (e.y >> 16);  // the number of planes is known now
   if (g.maskbits.size() >= ((size_t)1 << 31) || g.truns.size() >= ((size_t)1 << 31) ||
       g.centry.size() >= ((size_t)1 << 31))
@@ -2314,6 +2488,8 @@ int brkga_problem_create_multi(const BrkgaProblemDesc* descs, int32_t K, BrkgaPr
   pb->mach = g.mach;
   pb->tb.bsh = g.bsh;
   pb->tb.n_planes = g.n_planes;
+  pb->plain = g.bsh > 0;
+  for (const MachDev& m : g.mach) pb->plain = pb->plain && m.NW <= 32;
   for (const InstDev& id : g.inst) {
     int s2 = 1;
     while (s2 < id.N) s2 <<= 1;
