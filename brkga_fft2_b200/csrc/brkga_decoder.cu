@@ -1773,12 +1773,18 @@ int configure(BrkgaProblem* pb, int warps_req, int ctas_req, int plates_req) {
   const size_t grid_bytes = (size_t)grid_words * 4;
   // room of a plate in shared memory: its grid and two bytes a row
   const size_t slot_bytes = align_up((size_t)grid + (size_t)(Lmax + 1) / 2, 4) * 4;
-  cudaFuncAttributes fa4, fa2, fa1;
-  if (cudaFuncGetAttributes(&fa4, decode_form(pb, kForm4)) != cudaSuccess ||
-      cudaFuncGetAttributes(&fa2, decode_form(pb, kForm2)) != cudaSuccess ||
-      cudaFuncGetAttributes(&fa1, decode_form(pb, kForm1)) != cudaSuccess)
+  // Every kernel of a decode is looked up here, which loads it: a kernel first
+  // used by a launch is loaded inside that call.
+  cudaFuncAttributes fa[kForms], other;
+  for (int f = 0; f < kForms; ++f)
+    if (cudaFuncGetAttributes(&fa[f], decode_form(pb, (Form)f)) != cudaSuccess) return BRKGA_ERR_CUDA;
+  if (cudaFuncGetAttributes(&other, assign_sort_kernel) != cudaSuccess ||
+      cudaFuncGetAttributes(&other, order_items_kernel) != cudaSuccess ||
+      cudaFuncGetAttributes(&other, reduce_kernel) != cudaSuccess)
     return BRKGA_ERR_CUDA;
-  const size_t static_smem = std::max({fa4.sharedSizeBytes, fa2.sharedSizeBytes, fa1.sharedSizeBytes});
+  // the forms that may have plates in shared memory
+  const size_t static_smem =
+      std::max({fa[kForm4].sharedSizeBytes, fa[kForm2].sharedSizeBytes, fa[kForm1].sharedSizeBytes});
   const size_t per_sm = prop.sharedMemPerMultiprocessor;
   const size_t per_block_max = prop.sharedMemPerBlockOptin - static_smem;  // dynamic part
   const size_t reserve = 1024 + static_smem;  // per-block system reservation + static shared variables
