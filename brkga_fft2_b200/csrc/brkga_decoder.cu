@@ -85,12 +85,14 @@ constexpr unsigned long long kKeyNone = ~0ull;
 constexpr unsigned kFull = 0xFFFFFFFFu;
 
 struct RotDev {
-  int h, w, mw;      // rows, columns, 32-bit words per mask row
+  int h, w;          // rows, columns
+  short mw;          // 32-bit words per mask row
+  short gseg;        // pieces that groups of lanes test first (0: none, see group_segs())
   int trun, ntrun;   // runs of ones of all rows in test order: truns[trun .. trun + ntrun)
   int tseg, ntseg;   // the same runs in pieces of at most 32 columns: tsegs[tseg .. tseg + ntseg)
   int mask_base;     // first word in maskbits[] (h * mw words)
-  int gseg;          // pieces that groups of lanes test first (0: none, see group_segs())
 };
+static_assert(sizeof(RotDev) == 32, "RotDev layout");
 
 // The coarse test of one rotation at one alignment (its entries in centry[]
 // and cfilter[]); see coarse_ok() and coarse_and().
@@ -2076,7 +2078,7 @@ double coarse_tables(const BrkgaProblemDesc* descs, int K, Merged& g) {
           of_type[t].first += in_cores;
           of_type[t].second += rd.h;
         }
-        rd.gseg = group_segs(rd, g);
+        rd.gseg = (short)group_segs(rd, g);
         longest += rd.h;
       }
     for (int j = 0; j < d.n_genes; ++j) {
@@ -2189,7 +2191,7 @@ void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
         const uint8_t* mk = d->masks + d->rot_mask_offset[k];
         rd.h = h;
         rd.w = w;
-        rd.mw = (w + 31) / 32;
+        rd.mw = (short)((w + 31) / 32);
         rd.mask_base = (int)g.maskbits.size();
         int imax = 0, dmax = 0;  // row with the longest run of ones and that length
         runs.clear();
