@@ -116,7 +116,7 @@ static_assert(sizeof(RotList) == 16, "RotList layout");
 
 struct MachDev {
   int L, W, NW, RS;  // plate rows, columns, words per row, row stride (NW + 2 zero pad words)
-  int NB;            // blocks of rows
+  int NB;            // whole blocks of rows (the rows after them are in no core)
   double area;       // MachineData.bin_area
   double setup;      // MachineData.setup_time
 };
@@ -853,7 +853,7 @@ __device__ __forceinline__ unsigned long long search_plate(const Tables& tb, con
   return sh.best;
 }
 
-// The erosion planes and vacancies of blocks b0 .. b1 of a plate, from its
+// The erosion planes and vacancies of whole blocks b0 .. b1 of a plate, from its
 // rows.  A group of 8, 16 or 32 lanes takes a block, a lane one word of it (on
 // plates wider than 1024 columns a warp walks the row in steps that overlap by
 // the words an erosion reaches).  All threads of the CTA; no barrier.
@@ -868,7 +868,7 @@ __device__ __forceinline__ void update_blocks(const Tables& tb, const MachDev& m
     const int b = bb + (int)threadIdx.x / G;
     const bool on = b <= b1;
     const uint32_t* row = pr.grid + (size_t)(b << tb.bsh) * md.RS;
-    const int rows = min(1 << tb.bsh, md.L - (b << tb.bsh));
+    const int rows = min(1 << tb.bsh, md.L - (b << tb.bsh));  // 1 << bsh; written so it compiles 1 % faster
     for (int w0 = 0; w0 < md.NW; w0 += step) {
       const int w = w0 + gl;
       const uint32_t e0 = on && w < md.NW ? block_free(row, md.RS, md.W, rows, w) : 0u;
@@ -976,7 +976,7 @@ __device__ __forceinline__ void place_part(const Tables& tb, const MachDev& md, 
   }
   __syncthreads();
   if (!cells || by_rows) return;
-  update_blocks<kPlain>(tb, md, pr, ty >> tb.bsh, (ty + rd.h - 1) >> tb.bsh);
+  update_blocks<kPlain>(tb, md, pr, ty >> tb.bsh, min((ty + rd.h - 1) >> tb.bsh, md.NB - 1));
   __syncthreads();
 }
 
@@ -1541,10 +1541,13 @@ struct Shape {
 // library reserves it until the process exits.  Host code must not use the
 // symbol as an address; brkga_problem_create looks up its device address.
 // The tables and the pool plates' grids go into the first array, their erosion
-// planes and the CTAs' own plates into the second, which is large enough for as
-// many plates as the first can hold grids of (a plane set has four rows for
-// four or eight grid rows, and the CTAs' own grids are at most what shared
-// memory would hold, 34 MB).
+// planes and the CTAs' own plates into the second; the pool has as many plates
+// as both have room for.  The second does not limit it before the start of
+// another plate in the first: a plate's planes are at most as large as its grid
+// (four rows for a whole block of four or eight), so the CTAs' own plates take
+// at most twice the 31.5 MB of grids that shared memory would hold.  (With planes
+// for a block that is only begun, plates of 13 rows had room for 8,900 plates
+// instead of 10,600.)
 static __device__ __align__(256) unsigned char g_noalloc_scratch[BRKGA_NOALLOC_SCRATCH_BYTES];
 constexpr size_t kNoallocPlaneBytes = (size_t)2 * BRKGA_NOALLOC_SCRATCH_BYTES;
 static __device__ __align__(256) unsigned char g_noalloc_planes[kNoallocPlaneBytes];
@@ -1771,7 +1774,7 @@ int configure(BrkgaProblem* pb, int warps_req, int ctas_req, int plates_req) {
     planes = std::max(planes, pb->tb.n_planes * m.NB * m.RS);
   }
   const int grid_words = (int)align_up((size_t)grid, 4);
-  const int coarse_words = (int)align_up((size_t)planes + (size_t)(NBmax + 1) / 2, 4);
+  const int coarse_words = (int)std::max<size_t>(4, align_up((size_t)planes + (size_t)(NBmax + 1) / 2, 4));
   const size_t grid_bytes = (size_t)grid_words * 4;
   // room of a plate in shared memory: its grid and two bytes a row
   const size_t slot_bytes = align_up((size_t)grid + (size_t)(Lmax + 1) / 2, 4) * 4;
@@ -2086,7 +2089,7 @@ double coarse_tables(const BrkgaProblemDesc* descs, int K, Merged& g) {
       rows += of_type[d.gene_type[j]].second;
     }
   }
-  for (MachDev& m : g.mach) m.NB = (m.L + (1 << g.bsh) - 1) >> g.bsh;
+  for (MachDev& m : g.mach) m.NB = m.L >> g.bsh;
   return covered / rows;
 }
 
