@@ -1566,6 +1566,7 @@ struct BrkgaProblem {
   int task_max = kDefaultTaskMax;
   bool plain = false;  // the kernels' plain forms serve (see decode_kernel)
   Shape shape[3];      // 4, 2 and 1 warps per item
+  int64_t pool_per_cta = 0;  // plates an item may open (default_pool_bins())
   int min_S = 0;       // fewest own plates per CTA of the three shapes (pool sizing)
   int grid_words = 0, coarse_words = 0, vac_off = 0;  // words of a plate's grid, of its planes and vacancies, of the planes
   std::vector<MachDev> mach;
@@ -1692,8 +1693,43 @@ Layout layout_of(const BrkgaProblem* pb, const LaunchCounts& lc, int64_t pool_bi
   return l;
 }
 
+// Pool plates of a launch whose caller names no number: two an item, four where
+// some shape's CTAs have none of their own, as long as that is at most
+// pool_per_cta for every CTA that is resident.  A CTA keeps its pool plates for
+// its later items, so a launch of several waves needs as many as its resident
+// CTAs hold at most: there the pool and the CTAs' own plates take no more memory
+// than the grids alone of those two or four would, planes included.  (With planes
+// for all of them P100M4 4,000 rows took 1.43 GB, now 0.93; P400M8 4,096 rows 10.0
+// and 6.7; before the planes 0.97 and 6.8.)  A workspace sized for a population
+// serves every smaller one: the bytes never fall as the items grow.
 int64_t default_pool_bins(const BrkgaProblem* pb, int64_t items) {
-  return std::max<int64_t>(256, items * (pb->min_S > 0 ? 2 : 4));
+  const int64_t most = std::max<int64_t>(256, items * (pb->min_S > 0 ? 2 : 4));
+  const int64_t plate = pb->grid_words + pb->coarse_words;
+  const int64_t fit = (most * pb->grid_words - own_plates(pb, items) * plate) / plate;
+  return std::min(most, std::max(pb->pool_per_cta * scratch_slots(pb, items), fit));
+}
+
+// Plates an item may open, whatever its chromosome: all parts on the machine
+// that needs most for them, plates filled to kLeastFill at least, a plate for
+// each part that no second one like it fits beside; kPoolPerCta or more.
+constexpr double kLeastFill = 0.4;
+constexpr int kPoolPerCta = 16;
+int pool_per_cta(const BrkgaProblemDesc* descs, int K) {
+  double most = kPoolPerCta;
+  for (int k = 0; k < K; ++k) {
+    const BrkgaProblemDesc& d = descs[k];
+    for (int m = 0; m < d.n_machines; ++m) {
+      const double L = d.bin_length[m], W = d.bin_width[m];
+      double plates = 0.0;
+      for (int j = 0; j < d.n_genes; ++j) {
+        const int t = d.gene_type[j], r = t * 4 + d.part_best_rot[t];
+        const bool alone = 2 * std::min(d.rot_h[r], d.rot_w[r]) > std::max(L, W);
+        plates += alone ? 1.0 : std::min(1.0, d.part_area[t] / (kLeastFill * L * W));
+      }
+      most = std::max(most, plates);
+    }
+  }
+  return (int)std::ceil(std::min(most, (double)kMaxGenes));
 }
 
 template <typename T>
@@ -2499,6 +2535,7 @@ int brkga_problem_create_multi(const BrkgaProblemDesc* descs, int32_t K, BrkgaPr
   pb->mach = g.mach;
   pb->tb.bsh = g.bsh;
   pb->tb.n_planes = g.n_planes;
+  pb->pool_per_cta = pool_per_cta(descs, K);
   pb->plain = g.bsh > 0;
   for (const MachDev& m : g.mach) pb->plain = pb->plain && m.NW <= 32;
   for (const InstDev& id : g.inst) {
