@@ -1275,6 +1275,10 @@ struct GreedyArgs {
 // and their number.  In shared memory as long as it fits (up to some 8,000 parts).
 size_t greedy_state_bytes(int n, int M) { return (size_t)n * 28 + (size_t)M * 20; }
 constexpr size_t kGreedyMaxSmem = 229 * 1024;
+// Device memory of a call that stays with the problem: a grid and planes a part
+// (P100M4 2 MB, P400M8 30 MB).  More, at thousands of parts or plates of thousands
+// of cells, is given back by the call: beside so long a call an allocation is nothing.
+constexpr size_t kGreedyKeep = (size_t)64 << 20;
 
 __device__ __forceinline__ PlateRef greedy_plate(const GreedyArgs& g, int b) {
   uint32_t* planes = g.cpool + (size_t)b * g.coarse_words;
@@ -2824,7 +2828,7 @@ int brkga_initial_solution_host(BrkgaProblem* pb, const int32_t* h_order, int32_
   const bool in_smem = state_bytes <= kGreedyMaxSmem - 4096;
   const size_t off_state = o;
   if (!in_smem) o += kGreedyCtas * state_bytes;
-  if (o > pb->greedy_bytes) {  // kept for the next call on this problem
+  if (o > pb->greedy_bytes) {  // up to kGreedyKeep it is kept for the next call on this problem
     cudaFree(pb->greedy_ws);
     pb->greedy_ws = nullptr;
     pb->greedy_bytes = 0;
@@ -2887,6 +2891,11 @@ int brkga_initial_solution_host(BrkgaProblem* pb, const int32_t* h_order, int32_
         cudaMemcpy(h_machine_makespan, g.machine_makespan, (size_t)pb->M * 8, cudaMemcpyDeviceToHost) != cudaSuccess)
       st = BRKGA_ERR_CUDA;
   } while (false);
+  if (pb->greedy_bytes > kGreedyKeep) {
+    cudaFree(pb->greedy_ws);
+    pb->greedy_ws = nullptr;
+    pb->greedy_bytes = 0;
+  }
   return st;
 }
 

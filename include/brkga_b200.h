@@ -275,9 +275,9 @@ int brkga_last_counters(const BrkgaProblem* problem, int64_t* tests, int64_t* ch
  * makespan grows least — a new plate on a machine or any existing plate of it
  * that can take the part.  Outputs per placement, in order: h_machine[k] and
  * h_place[k] = (gene, plate index within the machine, x, bottom row y,
- * rotation); h_machine_makespan[M].  Synchronous; its device memory stays with
- * the problem for the next call.  Building the chromosome from this is host
- * work (brkga_fft2_b200.initial). */
+ * rotation); h_machine_makespan[M].  Synchronous; up to 64 MiB of its device
+ * memory stay with the problem for the next call, more is given back.  Building
+ * the chromosome from this is host work (brkga_fft2_b200.initial). */
 int brkga_initial_solution_host(BrkgaProblem* problem, const int32_t* h_order, int32_t n, int32_t* h_machine,
                                 BrkgaPlacement* h_place, double* h_machine_makespan);
 
