@@ -36,8 +36,10 @@ import numpy as np
 
 from . import abi
 
-# (warps per item, CTAs per SM, plates per item in shared memory)
-DEFAULT_SHAPES: Tuple[Tuple[int, int, int], ...] = ((4, 8, 0), (4, 8, 1), (4, 8, 2), (4, 6, 1), (4, 6, 2),
+# (warps per item, CTAs per SM, plates per item in shared memory).  The automatic shape is a candidate of its own: it
+# alone runs eight warps per item where a launch has at most one item per SM (P100M4, 20 rows: 0.436 ms against 0.52 of
+# the best explicit shape) and gives CTAs plates of their own without shared memory.
+DEFAULT_SHAPES: Tuple[Tuple[int, int, int], ...] = ((0, 0, -1), (4, 8, 0), (4, 8, 1), (4, 8, 2), (4, 6, 1), (4, 6, 2),
                                                     (2, 16, 0), (2, 16, 1), (2, 12, 1), (2, 12, 2), (2, 8, 2),
                                                     (1, 32, 0))
 DEFAULT_TASK_MAX: Tuple[int, ...] = (0, 64, 256, 1024, 8192)
@@ -76,7 +78,8 @@ def autotune(decoder, chrom, pops=None, shapes: Optional[Iterable[Tuple[int, int
     ``decoder`` is a ``DeviceDecoder`` (``chrom``: float32 CUDA [P, 2N]) or a
     ``MultiDecoder`` (``chrom``: the flat concatenated rows, ``pops``: rows per
     instance).  ``shapes`` are (warps per item, CTAs per SM, plates in shared
-    memory) triples; those that cannot be resident are skipped.  Returns
+    memory) triples, (0, 0, -1) the automatic one; those that cannot be resident
+    are skipped.  Returns
     ``{"key", "config": (warps, ctas_per_sm, smem_plates, task_max), "ms",
     "table": [(warps, ctas_per_sm, smem_plates, task_max, ms), ...],
     "cached"}`` and leaves the decoder on the chosen configuration.
