@@ -20,8 +20,8 @@ while the pairs are few, loses on wide plates with many surviving candidates
 ``autotune`` times the shapes first (``task_max`` at its default), then the
 ``task_max`` values at the best shape, each on the caller's own population
 (CUDA events around the decode kernel alone), keeps the fastest, and
-remembers it per device and grid size in a JSON cache, so later runs on the
-same plate grids skip the search.
+remembers it per device, grid size and library build in a JSON cache, so later
+runs on the same plate grids skip the search.
 
 The reference has no counterpart (its kernels use fixed launch shapes,
 full_native_decoder.py:2570-2755).
@@ -46,14 +46,15 @@ DEFAULT_TASK_MAX: Tuple[int, ...] = (0, 64, 256, 1024, 8192)
 
 
 def grid_key(packs: Sequence, device_index: int = 0) -> str:
-    """Cache key: device, SM count, the largest plate grid, genes and machines."""
+    """Cache key: device, SM count, the largest plate grid, genes and machines, and the library's build (other kernels
+    have other fastest shapes)."""
     import torch
     props = torch.cuda.get_device_properties(device_index)
     L = max(int(max(p.arrays["bin_length"])) for p in packs)
     W = max(int(max(p.arrays["bin_width"])) for p in packs)
     N = max(p.n_genes for p in packs)
     M = max(p.n_machines for p in packs)
-    return f"{props.name}|sm{props.multi_processor_count}|grid{L}x{W}|N{N}|M{M}|K{len(packs)}"
+    return f"{props.name}|sm{props.multi_processor_count}|grid{L}x{W}|N{N}|M{M}|K{len(packs)}|{abi.library_build_id()}"
 
 
 def _time_decode(decoder, run, repeats: int) -> float:

@@ -1,5 +1,6 @@
 """What the autotuner chooses from: the automatic launch shape is among its
-candidates, so that tuning never ends at something slower than not tuning."""
+candidates, so that tuning never ends at something slower than not tuning; and a
+cached choice belongs to one build of the library."""
 import types
 
 import numpy as np
@@ -18,7 +19,7 @@ def test_automatic_shape_is_a_candidate(monkeypatch):
             self.calls.append(cfg)
 
         def decode(self, chrom, out=None, kernel_events=None):
-            return out
+            return out.zero_()
 
         def launch_config(self):
             return self.calls[-1] if self.calls[-1][3] >= 0 else self.calls[-1][:3] + (0, 8192)
@@ -30,6 +31,19 @@ def test_automatic_shape_is_a_candidate(monkeypatch):
     res = at.autotune(dec, chrom, task_max_values=(), key="k")
     assert res["config"][:3] == (0, 0, -1) and res["ms"] == 1.0
     assert dec.calls[-1][:3] == (0, 0, -1)
+
+
+def test_key_belongs_to_a_build(monkeypatch):
+    import torch
+    monkeypatch.setattr(torch.cuda, "get_device_properties",
+                        lambda i: types.SimpleNamespace(name="dev", multi_processor_count=148))
+    pack = types.SimpleNamespace(arrays={"bin_length": np.array([300, 250]), "bin_width": np.array([300, 250])},
+                                 n_genes=100, n_machines=2)
+    keys = []
+    for build in ("a1", "b2"):
+        monkeypatch.setattr(at.abi, "library_build_id", lambda: build)
+        keys.append(at.grid_key([pack]))
+    assert keys[0] != keys[1] and all("grid300x300" in k for k in keys)
 
 
 @pytest.mark.gpu
