@@ -50,17 +50,18 @@ def encode(machine, place, instance_parts, type_ids, gene_type, nb_machines: int
     inst = np.asarray(instance_parts)
     N = inst.size
     array = np.zeros(2 * N)
-    free = {}  # genes of each part not yet used, the first one last
-    for idx in range(N - 1, -1, -1):
-        free.setdefault(int(inst[idx]), []).append(idx)
-    genes = place["gene"].tolist()
-    bins = place["bin"].tolist()
-    on = [[] for _ in range(nb_machines)]
+    free = {}  # genes of each part not yet used, the first one last; parts by their own values, whatever their type
+    for idx, part in reversed(list(enumerate(inst.tolist()))):
+        free.setdefault(part, []).append(idx)
+    if isinstance(place, np.ndarray):
+        genes, bins = place["gene"].tolist(), place["bin"].tolist()
+    else:
+        genes, bins = ([int(p[f]) for p in place] for f in ("gene", "bin"))
+    on = {}
     for k, m in enumerate(np.asarray(machine).tolist()):
-        if 0 <= m < nb_machines:
-            on[m].append(k)
+        on.setdefault(m, []).append(k)
     for m in range(nb_machines):
-        ks = sorted(on[m], key=lambda k: (bins[k], k))  # plates in creation order, parts in insertion order
+        ks = sorted(on.get(m, []), key=lambda k: (bins[k], k))  # plates in creation order, parts in insertion order
         left = [free.get(int(type_ids[gene_type[genes[k]]])) for k in ks]
         pos = np.array([f.pop() for f in left if f], dtype=np.int64)
         if nb_machines == 1:
