@@ -89,7 +89,7 @@ struct RotDev {
   short mw;          // 32-bit words per mask row
   short gseg;        // pieces that groups of lanes test first (0: none, see group_segs())
   int trun, ntrun;   // runs of ones of all rows in test order: truns[trun .. trun + ntrun)
-  int tseg, ntseg;   // the same runs in pieces of at most 32 columns: tsegs[tseg .. tseg + ntseg)
+  int tseg, ntseg;   // the same in pieces of at most 32 columns: truns[tseg .. tseg + ntseg), often the same list
   int mask_base;     // first word in maskbits[] (h * mw words)
 };
 static_assert(sizeof(RotDev) == 32, "RotDev layout");
@@ -151,8 +151,7 @@ struct Tables {
   const CoarseIdx* cidx;    // [rotation, indexed like rot][offset of the top row in a block]
   const uint2* centry;      // (first window's column | second one's << 16, plane row from the top row's block on)
   const uint32_t* cfilter;
-  const uint2* truns;       // (start | length << 16, row) per run of ones
-  const uint2* tsegs;       // the same, lengths at most 32
+  const uint2* truns;       // (start | length << 16, row) per run of ones, and per piece of one
   const uint32_t* maskbits;
   const uint8_t* newbin_ok;
   const uint8_t* fits;
@@ -763,7 +762,7 @@ __device__ __forceinline__ unsigned long long search_plate(const Tables& tb, con
     if (pass) surv[__popc(S & ((1u << lane) - 1u))] = (unsigned char)lane;
     __syncwarp();
     const unsigned inv = sh.inv[slot];
-    const uint2* segs = tb.tsegs + sh.rd[slot].tseg;
+    const uint2* segs = tb.truns + sh.rd[slot].tseg;
     const int nseg = sh.rd[slot].ntseg, gseg = kPlain ? kGroupSegs : sh.rd[slot].gseg;
     bool won = false;
     for (int t0 = 0; t0 < ntask && !won; t0 += 32) {
@@ -1590,7 +1589,6 @@ struct BrkgaProblem {
   uint2* d_centry = nullptr;
   uint32_t* d_cfilter = nullptr;
   uint2* d_truns = nullptr;
-  uint2* d_tsegs = nullptr;
   uint32_t* d_maskbits = nullptr;
   uint8_t* d_fits = nullptr;
   uint8_t* d_newbin_ok = nullptr;
@@ -1954,7 +1952,6 @@ struct Merged {
   std::vector<CoarseIdx> cidx;
   std::vector<uint2> centry;
   std::vector<uint32_t> cfilter;
-  std::vector<uint2> tsegs;
   int bsh = 0, n_planes = 0;  // rows of a block (2^bsh, 0: by rows), erosion planes that some core reads
   std::vector<std::pair<int, int>> longest;  // per mask row, rotation after rotation: [first, last + 1) of its longest run
   std::vector<int> n_runs;                   // per rotation: runs of ones of all rows
@@ -2011,7 +2008,7 @@ int group_segs(const RotDev& rd, const Merged& g) {
   if (rd.ntseg <= kGroupFewSegs) return 0;
   int cells = 0, q = 0;
   for (; q < rd.ntseg && q < kGroupMostSegs && (q < kGroupSegs || cells < kGroupCells); ++q)
-    cells += (int)(g.tsegs[rd.tseg + q].x >> 16);
+    cells += (int)(g.truns[rd.tseg + q].x >> 16);
   return q;
 }
 
@@ -2200,15 +2197,6 @@ uint32_t pack_cells(const uint8_t* cells, int n) {
   return v;
 }
 
-// First column from `at` on whose cell is set (or clear), w where there is none.
-int next_cell(const uint32_t* row, int w, int at, bool set) {
-  for (; at < w; at = (at | 31) + 1) {
-    const uint32_t v = (set ? row[at >> 5] : ~row[at >> 5]) >> (at & 31);
-    if (v) return std::min(w, at + __builtin_ctz(v));
-  }
-  return w;
-}
-
 // Append one instance: derived part tables (runs of ones, block cores,
 // bit-packed rows) with absolute indices, machines, times, flags.
 void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
@@ -2243,17 +2231,27 @@ void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
           const uint8_t* cells = mk + (size_t)i * w;
           for (int j = 0; j < w; j += 32) g.maskbits.push_back(pack_cells(cells + j, std::min(32, w - j)));
           const uint32_t* row = g.maskbits.data() + g.maskbits.size() - rd.mw;
-          int best = 0;
+          int best = 0, from = -1;  // from: first column of the run that is open
           g.longest.push_back({0, 0});
-          for (int j = next_cell(row, w, 0, true); j < w;) {
-            const int end = next_cell(row, w, j, false);
-            runs.push_back((uint32_t)j | ((uint32_t)(end - j) << 16));
-            if (end - j > best) {
-              best = end - j;
-              g.longest.back() = {j, end};
+          auto close = [&](int end) {
+            runs.push_back((uint32_t)from | ((uint32_t)(end - from) << 16));
+            if (end - from > best) {
+              best = end - from;
+              g.longest.back() = {from, end};
             }
-            j = next_cell(row, w, end, true);
+            from = -1;
+          };
+          uint32_t top = 0;  // the last word's highest cell
+          for (int wd = 0; wd < rd.mw; ++wd) {
+            // the columns at which a run begins or has ended, in turn
+            for (uint32_t edges = row[wd] ^ (row[wd] << 1 | top); edges; edges &= edges - 1) {
+              const int at = 32 * wd + __builtin_ctz(edges);
+              if (from < 0) from = at;
+              else close(at);
+            }
+            top = row[wd] >> 31;
           }
+          if (from >= 0) close(w);
           row_at.push_back((int)runs.size());
           if (best > dmax) {
             dmax = best;
@@ -2265,8 +2263,7 @@ void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
         // Plates fill from the bottom, so low rows reject a blocked candidate
         // soonest; spreading the first tests over the part's height catches
         // a collision higher up without walking every row below it.
-        rd.trun = (int)g.truns.size();
-        rd.tseg = (int)g.tsegs.size();
+        rd.tseg = (int)g.truns.size();
         {
           order.clear();
           used.assign(h, 0);
@@ -2280,18 +2277,26 @@ void merge_instance(const BrkgaProblemDesc* d, Merged& g) {
               }
           for (int i : order)
             for (int k = row_at[i]; k < row_at[i + 1]; ++k) {
-              const uint32_t r = runs[k];
-              g.truns.push_back(make_uint2(r, (unsigned)i));
-              const uint32_t s = r & 0xFFFFu, d = r >> 16;
+              const uint32_t s = runs[k] & 0xFFFFu, d = runs[k] >> 16;
               for (uint32_t at = 0; at < d; at += 32)
-                g.tsegs.push_back(make_uint2((s + at) | (std::min(32u, d - at) << 16), (unsigned)i));
+                g.truns.push_back(make_uint2((s + at) | (std::min(32u, d - at) << 16), (unsigned)i));
             }
+          rd.ntseg = (int)g.truns.size() - rd.tseg;
+          // Pieces are runs too, so one list serves where at most an eighth of it
+          // only continues a run; with two for every rotation, masks of many short
+          // runs took twice the memory (lattices of 200-800 cells 145 MB, now 80).
+          rd.trun = rd.tseg;
+          rd.ntrun = rd.ntseg;
+          if (rd.ntseg - (int)runs.size() > rd.ntseg / 8) {
+            rd.trun = (int)g.truns.size();
+            rd.ntrun = (int)runs.size();
+            for (int i : order)
+              for (int k = row_at[i]; k < row_at[i + 1]; ++k) g.truns.push_back(make_uint2(runs[k], (unsigned)i));
+          }
         }
-        rd.ntrun = (int)g.truns.size() - rd.trun;
-        rd.ntseg = (int)g.tsegs.size() - rd.tseg;
       }
       g.rot.push_back(rd);
-      g.n_runs.push_back(rd.ntrun);
+      g.n_runs.push_back(rd.h ? (int)runs.size() : 0);
     }
     g.area.push_back(d->part_area[t]);
     g.nrot.push_back(d->part_nrot[t]);
@@ -2560,7 +2565,7 @@ int brkga_problem_create_multi(const BrkgaProblemDesc* descs, int32_t K, BrkgaPr
       (st = upload(pb, &pb->d_pt, g.pt)) || (st = upload(pb, &pb->d_pth, g.pth)) ||
       (st = upload(pb, &pb->d_area, g.area)) || (st = upload(pb, &pb->d_nrot, g.nrot)) ||
       (st = upload(pb, &pb->d_best, g.best)) || (st = upload(pb, &pb->d_rot, g.rot)) ||
-      (st = upload(pb, &pb->d_tsegs, g.tsegs)) || (st = upload(pb, &pb->d_cidx, g.cidx)) ||
+      (st = upload(pb, &pb->d_cidx, g.cidx)) ||
       (st = upload(pb, &pb->d_centry, g.centry)) || (st = upload(pb, &pb->d_cfilter, g.cfilter)) || (st = upload(pb, &pb->d_truns, g.truns)) ||
       (st = upload(pb, &pb->d_maskbits, g.maskbits)) ||
       (st = upload(pb, &pb->d_fits, g.fits)) || (st = upload(pb, &pb->d_newbin_ok, g.newbin_ok)) ||
@@ -2584,7 +2589,6 @@ int brkga_problem_create_multi(const BrkgaProblemDesc* descs, int32_t K, BrkgaPr
   tb.centry = pb->d_centry;
   tb.cfilter = pb->d_cfilter;
   tb.truns = pb->d_truns;
-  tb.tsegs = pb->d_tsegs;
   tb.maskbits = pb->d_maskbits;
   tb.newbin_ok = pb->d_newbin_ok;
   tb.fits = pb->d_fits;
