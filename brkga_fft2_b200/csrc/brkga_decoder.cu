@@ -1971,8 +1971,12 @@ struct Merged {
 // full 2.6 / 2.8 ms (P200M6); 10-120 cell masks 5.8 / 6.5 ms (P100M4), 20-240
 // cell masks 20 / 26 ms (P400M8, 1,024 rows).  So four rows for small masks
 // and, up to medium ones, where the parts fill most of the plates.
-int block_shift(const BrkgaProblemDesc* descs, int K) {
-  double parts = 0.0, height = 0.0, fill = 0.0;  // over the genes: mean mask height, mean fill of their instance's plates
+constexpr double kMostlyFull = 0.6;
+struct MaskStats {
+  double height, fill;  // over the genes: mean mask height, mean fill of their instance's plates
+};
+MaskStats mask_stats(const BrkgaProblemDesc* descs, int K) {
+  double parts = 0.0, height = 0.0, fill = 0.0;
   for (int k = 0; k < K; ++k) {
     const BrkgaProblemDesc& d = descs[k];
     double area = 0.0, plates = 0.0;
@@ -1985,9 +1989,10 @@ int block_shift(const BrkgaProblemDesc* descs, int K) {
     parts += d.n_genes;
     fill += plates > 0.0 ? d.n_genes * area / plates : 0.0;
   }
-  if (height < 13.0 * parts) return 0;  // by rows, see coarse_blocks()
-  return height < 28.0 * parts || (height < 50.0 * parts && fill >= 0.6 * parts) ? 2 : 3;
+  return {height / parts, fill / parts};
 }
+
+int block_shift(const MaskStats& s) { return s.height < 28.0 || (s.height < 50.0 && s.fill >= kMostlyFull) ? 2 : 3; }
 
 // Where the test is by rows, a rotation's filter holds this many of its rows:
 // a tall, thin mask that passes 24 of them often fails at another one (200
@@ -2162,22 +2167,27 @@ double many_runs(const BrkgaProblemDesc* descs, int K, const Merged& g) {
 // tested by rows: the plate keeps the longest free run of every row instead of
 // planes, and a rotation's rows need one as long as their own longest run
 // (numba_utils.py:50-94).  By rows from a fifth of the mask rows in parts of many
-// runs on (frames, rings, H and U shapes have two runs at most), below 13 rows a
-// mask, and where less than 0.6 of the rows lie in cores at four rows a block.
-// One launch, by blocks / by rows:
+// runs on (frames, rings, H and U shapes have two runs at most), below ten rows a
+// mask, and where less than half of the rows lie in cores at four rows a block
+// (0.6 where the parts fill most of the plates; nearly empty plates let every row
+// through anyway).  One launch, by blocks as before / by rows:
 //   parts of 30-90 cells on three 300 x 300 plates, 500 rows: lattices 2.64 /
 //     0.85 ms, rectangles with holes 1.24 / 0.67, bars of 5 every 12-20 cells
 //     1.74 / 0.68; of solid parts and lattices 10 % lattices 0.79 / 0.86, 20 %
 //     1.02 / 0.89, 33 % 1.33 / 0.90; U shapes 1.18 / 1.73, frames of 4 cells
 //     0.81 / 1.27, solid parts (P100M4) 1.01 / 1.50;
-//   solid parts of 4-8 cells 1.53 / 1.20 ms, 5-15 1.92 / 1.66, 5-20 1.98 / 1.83,
-//     6-24 2.02 / 2.02, 14-25 1.08 / 1.29 (200 on three plates, 1,000 rows; the
-//     last 246 on two, 100 rows); rectangles of 4-12 cells 1.58 / 1.20, 1-3 x
-//     20-120 2.72 / 1.82 (2,000 rows).
-constexpr double kManyRunsShare = 0.2, kLeastCovered = 0.6;
+//   200 parts on three plates, 1,000 rows: of 4-8 cells on 50 x 50 1.53 / 1.20 ms,
+//     5-15 on 90 x 90 1.92 / 1.66, on 200 x 200 1.81 / 1.77, 5-20 on 120 x 120
+//     1.98 / 1.83, on 220 x 220 1.91 / 1.99, on 400 x 400 1.90 / 2.13, 6-24 on 150
+//     x 150 2.02 / 2.02, on 600 x 600 2.01 / 2.30; rectangles of 4-12 cells on 90 x
+//     90 1.58 / 1.20; 1-3 x 20-120 on 200 x 200, 2,000 rows, 2.72 / 1.82, 150 on
+//     600 x 600, 500 rows, 0.84 / 0.91.
+constexpr double kManyRunsShare = 0.2, kLeastHeight = 10.0, kNearlyEmpty = 0.03;
 void coarse_blocks(const BrkgaProblemDesc* descs, int K, Merged& g) {
-  g.bsh = many_runs(descs, K, g) > kManyRunsShare ? 0 : block_shift(descs, K);
-  while (coarse_tables(descs, K, g) < kLeastCovered && g.bsh) g.bsh = g.bsh == 3 ? 2 : 0;
+  const MaskStats s = mask_stats(descs, K);
+  g.bsh = many_runs(descs, K, g) > kManyRunsShare || s.height < kLeastHeight ? 0 : block_shift(s);
+  const double least = s.fill < kNearlyEmpty ? 0.0 : s.fill < kMostlyFull ? 0.5 : 0.6;
+  while (coarse_tables(descs, K, g) < least && g.bsh) g.bsh = g.bsh == 3 ? 2 : 0;
 }
 
 // A row's cells as bits, n <= 32 of them: eight bytes at a time, as (nonzero)
