@@ -4,10 +4,10 @@ The decode kernel has four knobs (``brkga_set_launch_config``).  Warps per
 item (1, 2 or 4) trade the latency of one (chromosome, machine) item against
 throughput: 4 finish an item sooner, 2 waste fewer lanes on speculative row
 chunks, so 2 win once the items fill several waves of resident CTAs, and 1
-(no CTA barrier at all) wins by 3 to 8 per cent once they fill some seven waves
-of 2-warp CTAs; the automatic choice follows these tiers (1 only from sixteen
-waves on, and 8 for a launch of at most one item per SM, which no explicit shape
-does).  More
+(no CTA barrier at all) wins once they fill about seven waves of 2-warp CTAs (by
+3 per cent at 4,000 P100M4 rows, 6.8 waves); the automatic choice follows these
+tiers (1 only from sixteen waves on, and 8 for a launch of at most one item per
+SM, which no explicit shape does).  More
 resident CTAs per SM hide more latency, plate grids in shared memory spare L1
 and L2 some of the searches' reads, and both draw on the same 228 KB of shared
 memory per SM, whose share per plate grows with the plate grid (a 500 x 500

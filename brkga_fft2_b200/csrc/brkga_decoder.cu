@@ -24,8 +24,8 @@
 //      shape), one (chromosome, machine) item at a time, longest first, from
 //      a device counter.  A plate is a grid of L rows of ceil(W/32)+2 32-bit
 //      words (bit x of a row = cell x) and the coarse data derived from it
-//      (erosion planes and longest free runs of blocks of rows, coarse_ok());
-//      each CTA has a few plates of its own, further ones come from a global
+//      (erosion planes and longest free runs of blocks of rows, or the longest
+//      free runs of the rows alone: coarse_ok(), coarse_blocks()); each CTA has a few plates of its own, further ones come from a global
 //      pool and stay with the CTA for its later items.  For each part:
 //      first-fit over plates (area filter, then the collision search), else a
 //      new plate with the best rotation at (0, L-1).  The collision search
@@ -80,7 +80,7 @@ constexpr int kCritSlots = 1024;  // per-SM marks, indexed by %smid
 // The coarse test's erosion planes: runs of 4, 8, 16 and 32 columns (see coarse_ok()).
 constexpr int kPlaneMin = 2;
 constexpr int kPlaneMax = 5;
-constexpr int kMaxTaskMax = 32 * 256;  // 32 candidates x the output words of the widest plate
+constexpr int kMaxTaskMax = 32 * 256;  // twice the pairs there can be: 32 candidates x 128 words of 64 columns
 constexpr unsigned long long kKeyNone = ~0ull;
 constexpr unsigned kFull = 0xFFFFFFFFu;
 
@@ -1251,8 +1251,8 @@ __global__ void reduce_kernel(const __grid_constant__ Tables tb, const __grid_co
 // one (the keys of alternate parts have buffers of their own, so none is
 // overwritten before every CTA has read it).  What bounds it is the latency of
 // one search and one insertion per part: the call took 7.4 ms on one CTA of
-// four warps with the search of runs and takes 1.65 ms here at 100 parts on four
-// machines (P100M4), 17.4 and 3.0 ms at 200 parts on six (P200M6), 1.34 and 0.70
+// four warps with the search of runs and takes 1.70 ms here at 100 parts on four
+// machines (P100M4), 17.4 and 3.2 ms at 200 parts on six (P200M6), 1.34 and 0.77
 // ms at 50 parts on two (P50M2).  Before the erosion planes, with four / eight /
 // sixteen warps per CTA: 2.9 / 2.4 / 2.35 ms, 5.5 / 4.9 / 4.9 and 1.05 / 0.94 /
 // 0.93 ms.
@@ -1797,7 +1797,8 @@ int occupancy(const BrkgaProblem* pb, int warps, size_t smem, int* occ) {
 // item): resident CTAs per SM and plates per item kept in shared memory.
 // For the requested CTA size (warps_req), ctas_req = 0 picks the CTAs
 // automatically (32 resident warps per SM, the register limit) and
-// plates_req = -1 keeps as many plates as fit in their share (at most 4);
+// plates_req = -1 keeps no grid in shared memory, but gives each CTA as many
+// plates of its own in the workspace as would fit in its share (at most 4);
 // the other CTA size, or both when warps_req = 0, gets the automatic shape.
 // A requested shape that cannot be resident is refused.
 int configure(BrkgaProblem* pb, int warps_req, int ctas_req, int plates_req) {

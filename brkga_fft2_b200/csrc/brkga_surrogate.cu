@@ -98,7 +98,7 @@ struct FeatParams {
   const int32_t* gene_type;
   const double* part_area;
   const double* pth;
-  const float4* shares;   // [machine * T + type], see ShareTable
+  const float4* shares;   // [machine * T + type], see share_table_kernel
   float inv_pth;          // 1 / max height time
   __nv_bfloat16* X;       // [rows, in_pad]
   int row_offset;

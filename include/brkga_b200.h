@@ -139,7 +139,8 @@ int brkga_decode_stage(int32_t stage, const BrkgaProblem* problem, const float* 
                        size_t ws_bytes, int64_t pool_bins, void* stream);
 
 /* Size of the library's fixed device scratch used by brkga_decode_noalloc:
- * 64 MiB, reserved on every GPU that loads the library until the process exits. */
+ * 64 MiB; with the planes' array beside it 192 MiB are reserved on every GPU that
+ * loads the library until the process exits. */
 #define BRKGA_NOALLOC_SCRATCH_BYTES (64u << 20)
 
 /* brkga_decode for callers that must not allocate device memory — code that
